@@ -66,10 +66,10 @@ __device__ __forceinline__ void lw_terms(float x, float& omt, float& fact, float
                          x * (1.f / 840.f))))));
     const float s_dfact = 0.5f + x * (-2.f / 3.f + x * (0.375f + x * (-2.f / 15.f + x * (5.f / 144.f +
                           x * (-1.f / 140.f + x * (49.f / 40320.f))))));
-    const float e = __expf(-x);
+    const float e = fast_exp(-x);
     const float e_omt = 1.f - e;
-    const float e_fact = __fdividef(e_omt, x) - e;
-    const float e_dfact = e - __fdividef(e_fact, x);
+    const float e_fact = fast_div(e_omt, x) - e;
+    const float e_dfact = e - fast_div(e_fact, x);
     const bool thin = x < 0.1f;
     omt = thin ? s_omt : e_omt;
     fact = thin ? s_fact : e_fact;

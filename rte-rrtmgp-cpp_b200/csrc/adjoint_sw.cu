@@ -97,7 +97,7 @@ __device__ __forceinline__ LocalAdj sw_local_adjoint(float tau, float w0, float 
     const float kk = 2.f * omw * kq;
     const bool kk_on = kk > 1.e-12f;
     const float kkc = fmaxf(kk, 1.e-12f);
-    const float rk = rsqrtf(kkc);   // 1 / k
+    const float rk = fast_rsqrt(kkc);   // 1 / k
     const float k = kkc * rk;
     float E1, e1, En, Tn;
     one_minus_exp(k * tau, E1, e1);
@@ -105,7 +105,7 @@ __device__ __forceinline__ LocalAdj sw_local_adjoint(float tau, float w0, float 
     const float E2 = E1 * (2.f - E1);
     const float e2 = e1 * e1;
     const float den = k * (1.f + e2) + g1 * E2;
-    const float rt = __fdividef(1.f, den);
+    const float rt = fast_div(1.f, den);
     const float km = k * mu0;
     const float fact = (1.f - km) * (1.f + km);
     const bool near1 = fabsf(fact) < 0.02f;   // k mu0 = 1 form (sw_layer_fast)
@@ -118,15 +118,15 @@ __device__ __forceinline__ LocalAdj sw_local_adjoint(float tau, float w0, float 
     float e1phi = 0.f, cI = 0.f, WI = 0.f, BR = 0.f, BT = 0.f;
     const float XI = a2 - k * km * g3, UI = a1 + k * km * g4, ZI = E1 * E1 + 2.f * e1 * En;
     if (near1) {
-        e1phi = xs ? e1 * ser : __fdividef(e1 - Tn, xi);
-        cI = __fdividef(w0 * rt, 1.f + km);
+        e1phi = xs ? e1 * ser : fast_div(e1 - Tn, xi);
+        cI = fast_div(w0 * rt, 1.f + km);
         WI = thick ? Tn * (1.f + e2) - 2.f * e1 : E1 * E1 - (1.f + e2) * En;
         BR = (a2 + k * g3) * ZI - 2.f * XI * e1 * e1phi * tmu;
         BT = 2.f * UI * e1phi * tmu + (a1 - k * g4) * WI;
         Rdir0 = cI * BR;
         Tdir0 = cI * BT;
     } else {
-        rt2 = __fdividef(w0 * rt, fact);
+        rt2 = fast_div(w0 * rt, fact);
         br = E2 * (a2 - k * km * g3) + k * (g3 - mu0 * a2) * (E1 * E1 + 2.f * (e1 * En));
         if (thick)
             bt = (1.f + km) * (a1 + k * g4) * Tn - (1.f - km) * (a1 - k * g4) * e2 * Tn - 2.f * ((k * g4 + a1 * km) * e1);
@@ -206,7 +206,7 @@ __device__ __forceinline__ LocalAdj sw_local_adjoint(float tau, float w0, float 
         }
         // divisions of the reverse mode as products with approximate reciprocals, like the
         // forward's __fdividef (an IEEE division is a multi-instruction sequence)
-        const float i1km = __fdividef(1.f, 1.f + km);
+        const float i1km = fast_div(1.f, 1.f + km);
         w0_b += c_b * rt * i1km;
         rt_b += c_b * w0 * i1km;
         km_b -= c_b * cI * i1km;
@@ -216,7 +216,7 @@ __device__ __forceinline__ LocalAdj sw_local_adjoint(float tau, float w0, float 
             e1_b += e1phi_b * ser;
             x_b = e1phi_b * e1 * dser;
         } else {
-            const float ixi = __fdividef(1.f, xi);
+            const float ixi = fast_div(1.f, xi);
             e1_b += e1phi_b * ixi;
             Tn_b -= e1phi_b * ixi;
             x_b = -e1phi_b * e1phi * ixi;
@@ -272,7 +272,7 @@ __device__ __forceinline__ LocalAdj sw_local_adjoint(float tau, float w0, float 
             En_b -= W2_b * (1.f + e2);
         }
         // rt2 = w0 rt / fact, fact = 1 - km^2
-        const float ifact = __fdividef(1.f, fact);
+        const float ifact = fast_div(1.f, fact);
         w0_b += rt2_b * rt * ifact;
         rt_b += rt2_b * w0 * ifact;
         const float fact_b = -rt2_b * rt2 * ifact;
@@ -323,8 +323,8 @@ __device__ __forceinline__ LocalAdj sw_local_adjoint(float tau, float w0, float 
     const bool okt = tau > 2.f * FLT_MIN;
     const float ts = w0 * tau;
     const bool oks = ts > 3.f * FLT_MIN;
-    const float itau = okt ? __fdividef(1.f, tau) : 0.f;
-    const float its = oks ? __fdividef(1.f, ts) : 0.f;
+    const float itau = okt ? fast_div(1.f, tau) : 0.f;
+    const float its = oks ? fast_div(1.f, ts) : 0.f;
     LocalAdj r;
     r.ta = taub - w0b * w0 * itau;
     r.tr = taub + w0b * omw * itau - gb * g * its;
@@ -440,11 +440,11 @@ __device__ __noinline__ LayerFwd sw_layer_forward(const float4* __restrict__ kma
     o.w0 = 0.f;
     o.omw = 1.f;
     if (o.tau > 2.f * FLT_MIN) {
-        const float inv = __fdividef(1.f, o.tau);
+        const float inv = fast_div(1.f, o.tau);
         o.w0 = ts * inv;
         o.omw = (ta + Rc->aux2) * inv;
     }
-    o.gasy = __fdividef(Rc->aux.w, fmaxf(ts, 3.f * FLT_MIN));
+    o.gasy = fast_div(Rc->aux.w, fmaxf(ts, 3.f * FLT_MIN));
     sw_layer_fast(o.tau, o.w0, o.omw, o.gasy, mu0, mu0_inv, o.R, o.T, o.Rdir, o.Tdir, o.Tn, o.adif, o.adir);
     return o;
 }
@@ -716,7 +716,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             vR[i] = R; vT[i] = T; vRd[i] = Rdir; vTd[i] = Tdir; vTn[i] = Tn; vAf[i] = adif; vAr[i] = adir;
             vP[i] = P;
             const float su = Rdir * P, sd = Tdir * P;
-            const float den = __fdividef(1.f, fmaf(-cRd, R, 1.f));
+            const float den = fast_div(1.f, fmaf(-cRd, R, 1.f));
             const float nRu = cRu + cT * cT * R * den;
             const float nRd = R + T * T * cRd * den;
             const float nU = cU + cT * (su + R * cD) * den;
@@ -752,7 +752,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             }
             const float4 m = sm_x2a[c * 32 + lane];
             const float Dc = sm_x2b[c * 32 + lane];
-            const float den = __fdividef(1.f, fmaf(-m.y, alb, 1.f));
+            const float den = fast_div(1.f, fmaf(-m.y, alb, 1.f));
             if (c < Wg) {
                 const float F = m.z * den, G = fmaf(m.y, src, Dc) * den;
                 fb = fmaf(fa, G, fb);
@@ -774,7 +774,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
 #pragma unroll
             for (int i = CL - 1; i >= 0; --i) {
                 const float su = vRd[i] * vDir[i], sd = vTd[i] * vDir[i];
-                const float den = __fdividef(1.f, fmaf(-vR[i], a, 1.f));
+                const float den = fast_div(1.f, fmaf(-vR[i], a, 1.f));
                 const float na = vR[i] + vT[i] * vT[i] * a * den;
                 const float ns = su + vT[i] * fmaf(a, sd, s) * den;
                 vA[i] = na;
@@ -791,7 +791,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             vFd[i] = fd;
             const float a_n = (i + 1 < CL) ? vA[i + 1] : alb_in;
             const float s_n = (i + 1 < CL) ? vS[i + 1] : src_in;
-            const float den = __fdividef(1.f, fmaf(-vR[i], a_n, 1.f));
+            const float den = fast_div(1.f, fmaf(-vR[i], a_n, 1.f));
             fd = (vT[i] * fd + vR[i] * s_n + vTd[i] * vDir[i]) * den;
         }
         const float fd_bot = fd;
@@ -835,7 +835,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             for (int i = CL - 1; i >= 0; --i) {
                 const int jl = w * CL + i;
                 const float a_n = (i + 1 < CL) ? vA[i + 1] : alb_in;
-                const float den = __fdividef(1.f, fmaf(-vR[i], a_n, 1.f));
+                const float den = fast_div(1.f, fmaf(-vR[i], a_n, 1.f));
                 const float c = vT[i] * den;
                 const float h = sm_hh[jl];
                 const float off = c * h * vAf[i] * a_n + sm_be[jl] + h * vAf[i] + sm_al[jl] * vA[i];
@@ -856,7 +856,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
         for (int i = CL - 1; i >= 0; --i) {
             const int jl = w * CL + i;
             const float a_n = (i + 1 < CL) ? vA[i + 1] : alb_in;
-            const float den = __fdividef(1.f, fmaf(-vR[i], a_n, 1.f));
+            const float den = fast_div(1.f, fmaf(-vR[i], a_n, 1.f));
             const float h = sm_hh[jl];
             const float Fc = Fraw + h * vAf[i] * a_n;
             vFc[i] = Fc;
@@ -872,7 +872,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
                 const float a_n = (i + 1 < CL) ? vA[i + 1] : alb_in;
                 const float s_n = (i + 1 < CL) ? vS[i + 1] : src_in;
                 const float fd_n = (i + 1 < CL) ? vFd[i + 1] : fd_bot;
-                const float den = __fdividef(1.f, fmaf(-vR[i], a_n, 1.f));
+                const float den = fast_div(1.f, fmaf(-vR[i], a_n, 1.f));
                 const float td = vT[i] * den;
                 const float ub = sm_al[jl + 1] + sm_hh[jl] * vAf[i];
                 const float p = td * td, q = td * den * (vTd[i] * vDir[i] + vR[i] * s_n), r = td;
@@ -907,7 +907,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
                 const float a_n = (i + 1 < CL) ? vA[i + 1] : alb_in;
                 const float s_n = (i + 1 < CL) ? vS[i + 1] : src_in;
                 const float fd_n = (i + 1 < CL) ? vFd[i + 1] : fd_bot;
-                const float den = __fdividef(1.f, fmaf(-vR[i], a_n, 1.f));
+                const float den = fast_div(1.f, fmaf(-vR[i], a_n, 1.f));
                 const float T = vT[i], R = vR[i], sdn = vTd[i] * vDir[i], Fc = vFc[i];
                 const float num_fd = T * vFd[i] + R * s_n + sdn;              // fd_(i+1) / den
                 const float denb = A_ * T * T * a_n + S_ * T * (s_n + a_n * sdn) + Fc * num_fd;

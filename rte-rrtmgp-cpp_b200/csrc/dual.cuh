@@ -96,8 +96,8 @@ template <int N>
 __device__ __forceinline__ Dual<N> ddiv(const Dual<N>& a, const Dual<N>& b, bool fast)
 {
     Dual<N> r;
-    const float ib = fast ? __fdividef(1.f, b.v) : 1.f / b.v;
-    r.v = fast ? __fdividef(a.v, b.v) : a.v / b.v;
+    const float ib = fast ? fast_div(1.f, b.v) : 1.f / b.v;
+    r.v = fast ? fast_div(a.v, b.v) : a.v / b.v;
 #pragma unroll
     for (int i = 0; i < N; ++i) r.d[i] = (a.d[i] - r.v * b.d[i]) * ib;
     return r;

@@ -305,7 +305,7 @@ gas_optics_sw_packed_kernel(const KdistView<float> k, const GasSet<float> gases,
             const Idx o = cl + Idx(g) * ncl;
             tau[o] = tt;
             // approximate division (2 ulp for normal divisors; tt is far below 2^126)
-            ssa[o] = tt > two_tmin ? __fdividef(tr, tt) : 0.f;
+            ssa[o] = tt > two_tmin ? fast_div(tr, tt) : 0.f;
             gasy[o] = 0.f;
         }
     }

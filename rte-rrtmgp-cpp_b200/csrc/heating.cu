@@ -38,7 +38,7 @@ template <>
 __device__ __forceinline__ void lw_layer_terms<float>(float tau, float D, float lay, float ldn, float lup, float& omt,
                                                       float& sdn, float& sup)
 {
-    lw_layer_fast(tau, D, lay, ldn, lup, omt, sdn, sup);
+    lw_layer_fast<false>(tau, D, lay, ldn, lup, omt, sdn, sup);
 }
 template <>
 __device__ __forceinline__ void lw_layer_terms<double>(double tau, double D, double lay, double ldn, double lup,

@@ -498,7 +498,7 @@ __device__ __forceinline__ void sw_layer_coeffs_abs(float tau, float ssa, float 
 template <typename T>
 __device__ __forceinline__ T adding_den(T R, T a) { return T(1) / (T(1) - R * a); }
 template <>
-__device__ __forceinline__ float adding_den<float>(float R, float a) { return __fdividef(1.f, fmaf(-R, a, 1.f)); }
+__device__ __forceinline__ float adding_den<float>(float R, float a) { return fast_div(1.f, fmaf(-R, a, 1.f)); }
 
 // Arguments of the chunked shortwave solvers other than the layer optical properties.
 template <typename T>

@@ -7,6 +7,31 @@
 
 namespace rrtmgp_b200 {
 
+// Approximate FP32 division, reciprocal square root and exponential that flush subnormal operands
+// and results to zero.  In the normal range they are what __fdividef, rsqrtf and __expf compute;
+// those also carry subnormals, which takes a compare and two scalings per call -- 8 divisions,
+// two exponentials and a root per (layer, g-point) in the shortwave -- although every
+// divisor here is kept normal by a guard (or its quotient is discarded by a select), and a
+// transmissivity or flux fraction below 1.2e-38 is zero at any output's precision.
+__device__ __forceinline__ float fast_div(float a, float b)
+{
+    float r;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float fast_rsqrt(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float fast_exp(float x)
+{
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));
+    return r;
+}
+
 // Gauss-Jacobi secants and weights of Rte_lw::rte_lw (src/Rte_lw.cpp:101-113), row n-1 for
 // n quadrature angles.
 __device__ __constant__ static const double kGaussDs[4][4] = {
@@ -57,23 +82,28 @@ __device__ __forceinline__ void lw_thin_terms(float tl, float& omt, float& fact)
     fact = tl * (0.5f + tl * (-1.f / 3.f + tl * (0.125f + tl * (-1.f / 30.f + tl * (1.f / 144.f -
            tl * (1.f / 840.f))))));
 }
+// FLUSH: the subnormal-flushing forms (fast_exp, fast_div).  The fused kernels use them (8192 x 128
+// forward 3.01 -> 2.96 ms); the per-stage kernels are not faster with them, and
+// heating_rate_lw_layers is slower (4096 x 91: 430 -> 483 us).
+template <bool FLUSH>
 __device__ __forceinline__ void lw_thick_terms(float tl, float& omt, float& fact)
 {
-    const float trans = __expf(-tl);
+    const float trans = FLUSH ? fast_exp(-tl) : __expf(-tl);
     omt = 1.f - trans;
-    fact = __fdividef(omt, tl) - trans;
+    fact = (FLUSH ? fast_div(omt, tl) : __fdividef(omt, tl)) - trans;
 }
 
 // Layer transmissivity complement and sources in FP32 for the fused kernels, whose lanes are
 // g-points of one layer (thin and thick layers mix within a warp): both forms are evaluated
 // and one is selected, so the warp does not diverge.
+template <bool FLUSH = true>
 __device__ __forceinline__ void lw_layer_fast(float tau, float D, float lay, float ldn, float lup, float& omt,
                                               float& sdn, float& sup)
 {
     const float tl = tau * D;
     float s_omt, s_fact, e_omt, e_fact;
     lw_thin_terms(tl, s_omt, s_fact);
-    lw_thick_terms(tl, e_omt, e_fact);
+    lw_thick_terms<FLUSH>(tl, e_omt, e_fact);
     const bool thin = tl < 0.1f;
     omt = thin ? s_omt : e_omt;
     const float fact = thin ? s_fact : e_fact;
@@ -92,7 +122,7 @@ __device__ __forceinline__ void lw_layer<float>(float tau, float D, float lay, f
     if (tl < 0.1f)
         lw_thin_terms(tl, omt, fact);
     else
-        lw_thick_terms(tl, omt, fact);
+        lw_thick_terms<false>(tl, omt, fact);
     trans = 1.f - omt;
     src_dn = omt * lev_dn + 2.f * fact * (lay - lev_dn);
     src_up = omt * lev_up + 2.f * fact * (lay - lev_up);

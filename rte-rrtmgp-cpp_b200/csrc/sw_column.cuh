@@ -167,11 +167,11 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
                 const float ts = tr + Rc.aux.z;
                 float w0 = 0.f, omw = 1.f;
                 if (tau > 2.f * FLT_MIN) {
-                    const float inv = __fdividef(1.f, tau);
+                    const float inv = fast_div(1.f, tau);
                     w0 = ts * inv;
                     omw = (ta + Rc.aux2) * inv;
                 }
-                const float gasy = __fdividef(Rc.aux.w, fmaxf(ts, 3.f * FLT_MIN));
+                const float gasy = fast_div(Rc.aux.w, fmaxf(ts, 3.f * FLT_MIN));
                 sw_layer_fast(tau, w0, omw, gasy, mu0, mu0_inv, R, T, Rdir, Tdir, Tn, adif, adir);
             }
             vR[i] = R;
@@ -182,7 +182,7 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
             vAd[i] = adif;
             vAdir[i] = adir * P;
             // Add layer i below the composite of layers 0..i-1.
-            const float den = __fdividef(1.f, fmaf(-cRd, R, 1.f));
+            const float den = fast_div(1.f, fmaf(-cRd, R, 1.f));
             const float nRu = cRu + cT * cT * R * den;
             const float nRd = R + T * T * cRd * den;
             const float nU = cU + cT * (vSu[i] + R * cD) * den;
@@ -233,7 +233,7 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
             for (int c = NW - 1; c >= 0; --c) {
                 const float4 m = sm_comp[c * 32 + lane];
                 const float D = sm_compd[c * 32 + lane];
-                const float den = __fdividef(1.f, fmaf(-m.y, alb, 1.f));
+                const float den = fast_div(1.f, fmaf(-m.y, alb, 1.f));
                 cx.put(&sm_comp[c * 32 + lane], make_float4(alb, src, m.z * den, fmaf(m.y, src, D) * den));
                 const float nalb = m.x + m.z * m.z * alb * den;
                 src = m.w + m.z * fmaf(alb, D, src) * den;
@@ -257,7 +257,7 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
 #pragma unroll
             for (int i = CL - 1; i >= 0; --i) {
                 const float su = vSu[i] * dtop, sd = vSd[i] * dtop;
-                const float den = __fdividef(1.f, fmaf(-vR[i], a, 1.f));
+                const float den = fast_div(1.f, fmaf(-vR[i], a, 1.f));
                 const float na = vR[i] + vT[i] * vT[i] * a * den;
                 const float ns = su + vT[i] * fmaf(a, sd, s) * den;
                 vSd[i] = sd;
@@ -275,7 +275,7 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
             const float a_n = (i + 1 < CL) ? vA[i + 1] : alb_in;
             const float s_n = (i + 1 < CL) ? vSu[i + 1] : src_in;
             const float fu = fmaf(fd, vA[i], vSu[i]);
-            const float den = __fdividef(1.f, fmaf(-vR[i], a_n, 1.f));
+            const float den = fast_div(1.f, fmaf(-vR[i], a_n, 1.f));
             const float fdn = (vT[i] * fd + vR[i] * s_n + vSd[i]) * den;
             const float fun = fmaf(fdn, a_n, s_n);
             vUp[i] = fu;

@@ -64,7 +64,7 @@ __device__ __forceinline__ void one_minus_exp(float x, float& E, float& e)
 {
     const float Es = x * (1.f - x * (1.f / 2.f - x * (1.f / 6.f - x * (1.f / 24.f - x * (1.f / 120.f - x * (1.f / 720.f -
                      x * (1.f / 5040.f - x * (1.f / 40320.f))))))));
-    const float ex = __expf(-x);
+    const float ex = fast_exp(-x);
     const bool small = x < 0.5f;
     E = small ? Es : 1.f - ex;
     e = small ? 1.f - Es : ex;
@@ -105,13 +105,13 @@ __device__ __forceinline__ void sw_layer_fast(float tau, float w0, float omw, fl
     const float a2 = g1 * g3 + g2 * g4;
     const float kk = 2.f * omw * (2.f - .5f * w0 * (1.f + 3.f * g));
     const float kkc = fmaxf(kk, 1.e-12f);
-    const float k = kkc * rsqrtf(kkc);
+    const float k = kkc * fast_rsqrt(kkc);
     float E1, e1, En;
     one_minus_exp(k * tau, E1, e1);
     one_minus_exp(tau * mu0_inv, En, Tn);
     const float E2 = E1 * (2.f - E1);
     const float e2 = e1 * e1;
-    const float rt = __fdividef(1.f, k * (1.f + e2) + g1 * E2);
+    const float rt = fast_div(1.f, k * (1.f + e2) + g1 * E2);
     R = rt * g2 * E2;
     T = rt * 2.f * k * e1;
     adif = rt * (k * E1 * E1 + 2.f * omw * E2);
@@ -123,13 +123,13 @@ __device__ __forceinline__ void sw_layer_fast(float tau, float w0, float omw, fl
         const float tm = tau * mu0_inv;
         const float x = tm * (1.f - km);
         const float ser = 1.f - x * (.5f - x * (1.f / 6.f - x * (1.f / 24.f - x * (1.f / 120.f))));
-        const float e1phi = fabsf(x) < .5f ? e1 * ser : __fdividef(e1 - Tn, x);
-        const float c = __fdividef(w0 * rt, 1.f + km);
+        const float e1phi = fabsf(x) < .5f ? e1 * ser : fast_div(e1 - Tn, x);
+        const float c = fast_div(w0 * rt, 1.f + km);
         const float W = thick ? Tn * (1.f + e2) - 2.f * e1 : E1 * E1 - (1.f + e2) * En;
         Rdir0 = c * ((a2 + k * g3) * (E1 * E1 + 2.f * e1 * En) - 2.f * (a2 - k * km * g3) * e1 * e1phi * tm);
         Tdir0 = c * (2.f * (a1 + k * km * g4) * e1phi * tm + (a1 - k * g4) * W);
     } else {
-        const float rt2 = __fdividef(w0 * rt, fact);
+        const float rt2 = fast_div(w0 * rt, fact);
         const float br = E2 * (a2 - k * km * g3) + k * (g3 - mu0 * a2) * (E1 * E1 + 2.f * e1 * En);
         const float bt_thick =
             (1.f + km) * (a1 + k * g4) * Tn - (1.f - km) * (a1 - k * g4) * e2 * Tn - 2.f * (k * g4 + a1 * km) * e1;
