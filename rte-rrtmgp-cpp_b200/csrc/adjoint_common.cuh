@@ -33,24 +33,19 @@ namespace rrtmgp_b200 {
 namespace fused {
 
 struct __align__(16) DRec {
-    float4 wT0, wT1;    // d tau_major / dT on kmaj4 rows 0 / 1
+    float4 wT0, wT1;    // d tau_major / dT on kmaj4 / kmp8 rows 0 / 1
     float4 wH0, wH1;    // d tau_major / d vmr_h2o
     float4 wO0, wO1;    // d tau_major / d vmr_o3
-    float4 pT0, pT1;    // d pfrac / dT on pfrac4 rows (LW; unused in SW)
+    float4 pT0, pT1;    // d pfrac / dT on kmp8 rows (LW; unused in SW)
     float4 pH0, pH1;
     float4 pO0, pO1;
     float4 fmT, fmH, fmO;   // d fminor / dx on the minor corners (lo.x, lo.y, hi.x, hi.y)
     float4 dB;              // LW: dB/dT of the band Planck function at T_lay, T_top, T_bot, T_sfc
                             // SW: d col_rayl / d vmr_h2o in x
     float4 pad;             // 272 bytes: an odd number of 16-byte units (bank-conflict-free stores
-                            // of consecutive records, as Rec)
+                            // of consecutive records, as LwRec)
 };                          // (minor scalings and their derivatives: layer_minor_scalings_d)
 static_assert(sizeof(DRec) == 272, "DRec stride");
-
-__device__ __forceinline__ float dot4(const float4& a, const float4& b)
-{
-    return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
-}
 
 // Slope of the piecewise-linear interpolate1D table at val.
 __device__ __forceinline__ float interpolate1D_slope(float val, float offset, float delta, int len,
@@ -196,37 +191,24 @@ __device__ __forceinline__ void layer_minor_scalings_d(const KdistView<float>& k
     }
 }
 
-// Adjoint of tau_abs for g-point g: accumulates tau_bar * dtau/dx into gT, gH, gO.  c0, c1:
-// the g-point's kmaj4 corners of the record's two rows (loaded by the caller, early); sc4:
-// the layer's scaling table (layer_minor_scalings_d).  DENSE as tau_abs.
-template <bool DENSE = false>
-__device__ __forceinline__ void tau_abs_adjoint(const KdistView<float>& k, const Rec& R, const DRec& D, int g,
-                                                int4 mg, int nmax, float tb, const float4& c0, const float4& c1,
-                                                const float4* sc4, float& gT, float& gH, float& gO)
+// Adjoint of tau_abs for g-point g: accumulates tau_bar * dtau/dx into gT, gH, gO.  r: load_rows
+// of the record (by the caller, early); sc4: the layer's scaling table (layer_minor_scalings_d).
+// The rest as tau_abs.
+template <bool SW, bool DENSE, class Rec>
+__device__ __forceinline__ void tau_abs_adjoint(const GasTab& k, const Rec& R, const DRec& D, int a, int g,
+                                                const GasRows& r, const MinorRef& m, float tb, const float4* sc4,
+                                                float& gT, float& gH, float& gO)
 {
-    float dT = dot4(D.wT0, c0) + dot4(D.wT1, c1);
-    float dH = dot4(D.wH0, c0) + dot4(D.wH1, c1);
-    float dO = dot4(D.wO0, c0) + dot4(D.wO1, c1);
-    const float2* kn = k.kmin2[R.a];
-    auto term = [&](int code, bool on) {
-        const int c = code >> kScalBits;
-        const float2 lo = __ldg(kn + (R.kb.z + c));
-        const float2 hi = __ldg(kn + (R.kb.w + c));
-        const float4 cr = make_float4(lo.x, lo.y, hi.x, hi.y);
+    float dT = dot4(D.wT0, r.c0) + dot4(D.wT1, r.c1);
+    float dH = dot4(D.wH0, r.c0) + dot4(D.wH1, r.c1);
+    float dO = dot4(D.wO0, r.c0) + dot4(D.wO1, r.c1);
+    for_minors<SW, DENSE>(k, R.kb, a, g, r, m, [&](const float4& cr, int sid) {
         const float M = dot4(R.fm, cr);
-        const float4 S = sc4[code & (kMaxScal - 1)];
-        const float tT = S.x * (S.y * M + dot4(D.fmT, cr));
-        const float tH = S.z * M + S.x * dot4(D.fmH, cr);
-        const float tO = S.w * M + S.x * dot4(D.fmO, cr);
-        dT += on ? tT : 0.f;
-        dH += on ? tH : 0.f;
-        dO += on ? tO : 0.f;
-    };
-#pragma unroll
-    for (int n = 0; n < 3; ++n)
-        if (n < nmax) term(n == 0 ? mg.y : (n == 1 ? mg.z : mg.w), n < mg.x);
-    if constexpr (DENSE)
-        for (int n = 3; n < nmax; ++n) term(minor_code_at(k, R.a, mg, g, n), n < mg.x);
+        const float4 S = sc4[sid];   // scaling, d ln / dT, d / d h2o, d / d o3
+        dT += S.x * (S.y * M + dot4(D.fmT, cr));
+        dH += S.z * M + S.x * dot4(D.fmH, cr);
+        dO += S.w * M + S.x * dot4(D.fmO, cr);
+    });
     gT += tb * dT;
     gH += tb * dH;
     gO += tb * dO;

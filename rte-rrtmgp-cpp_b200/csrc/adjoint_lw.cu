@@ -133,7 +133,7 @@ __host__ __device__ __forceinline__ AdjLayout adj_layout(int LPC, int ngas, int 
     L.maps = align16(L.levbot + sizeof(double) * 16);
     L.sfc = align16(L.maps + sizeof(float4) * size_t(NWt) * 32 * 2 * nbuf);
     L.recs = align16(L.sfc + sizeof(float) * 32 * nbuf);
-    L.drecs = align16(L.recs + sizeof(Rec) * size_t(NWc) * CL * mgb);
+    L.drecs = align16(L.recs + sizeof(LwRec) * size_t(NWc) * CL * mgb);
     L.total = align16(L.drecs + sizeof(DRec) * size_t(NWc) * CL * mgb);
     return L;
 }
@@ -189,7 +189,7 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
     double* sm_levbot = reinterpret_cast<double*>(smem_raw + SL.levbot);
     float4* const sm_map0 = reinterpret_cast<float4*>(smem_raw + SL.maps);
     float* const sm_sfc0 = reinterpret_cast<float*>(smem_raw + SL.sfc);
-    Rec* recs = reinterpret_cast<Rec*>(smem_raw + SL.recs) + w * CL * mgb;
+    LwRec* recs = reinterpret_cast<LwRec*>(smem_raw + SL.recs) + w * CL * mgb;
     DRec* drecs = reinterpret_cast<DRec*>(smem_raw + SL.drecs) + w * CL * mgb;
     auto at_rank = [&](auto* p, int rr) { return CLUSTER ? remote(cluster, p, rr) : p; };
     auto csync = [&]() {
@@ -240,6 +240,10 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
     }
     __syncthreads();
 
+    // bit i: layer i of this warp's chunk is in the upper atmosphere
+    const unsigned upper = __ballot_sync(0xffffffffu, lane < CL && j0 + w * CL + lane < nlay &&
+                                                          st[w * CL + (lane < CL ? lane : 0)].itropo);
+
     const float D = 1.66f;
     const int ngpt = k.ngpt;
     const int L_end = NWt * CL;
@@ -265,10 +269,7 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
         const int b0 = k.group_band0[gg];
         const int gband = gv ? k.gpt2band[g] : b0;
         const int slot = gband - b0;
-        const int4 mg0 = minor_entry(k.minor_g[0], g, gv);
-        const int4 mg1 = minor_entry(k.minor_g[1], g, gv);
-        const int nm0 = __reduce_max_sync(0xffffffffu, mg0.x);
-        const int nm1 = __reduce_max_sync(0xffffffffu, mg1.x);
+        const MinorRef mr0 = minor_ref(k, 0, g, gv), mr1 = minor_ref(k, 1, g, gv);
         const float emis = gv ? __ldg(sfc_emis + gband + size_t(icol) * nband) : 0.f;
 
         for (int r = lane; r < CL * mgb; r += 32) {
@@ -276,17 +277,17 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
             const int jj = j0 + jl;
             const int b = b0 + r / CL;
             if (jj < nlay && b < nband && k.band_lims[2 * b] < 32 * gg + 32) {
-                Rec& R = recs[r];
+                LwRec& R = recs[r];
                 DRec& DR = drecs[r];
                 const LayerState s = st[jl];
-                record_weights(k, R, s, sm_cg + jl, LPC, b);
                 const float* tp = k.totplnk + size_t(b) * k.nplanck;
                 const bool bottom = jj == nlay - 1;
+                record_weights(k, R, s, sm_cg + jl, LPC, b,
+                               bottom ? interpolate1D(ts, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp) : 0.f);
                 R.aux = make_float4(interpolate1D(s.t, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp),
                                     interpolate1D(s.t_top, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp),
                                     interpolate1D(s.t_bot, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp),
                                     sm_cld[b * LPC + jl]);
-                R.aux2 = bottom ? interpolate1D(ts, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp) : 0.f;
                 build_drec(k, DR, s, sm_cg + jl, LPC, b, idx_o3, cd_internal);
                 DR.dB = make_float4(interpolate1D_slope(s.t, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp),
                                     interpolate1D_slope(s.t_top, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp),
@@ -307,17 +308,19 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
             const int j = j0 + jl;
             vtau[i] = 0.f; vpf[i] = 0.f; omt[i] = 0.f; sdn[i] = 0.f; sup[i] = 0.f;
             if (j < nlay && gv) {
-                const Rec& R = recs[slot * CL + i];
-                const float tau = tau_abs<DENSE>(k, R, g, R.a ? mg1 : mg0, R.a ? nm1 : nm0,
-                                          &sm_sc4[jl * k.max_nscal].x, 4) + R.aux.w;
-                const float4 p0 = __ldg(k.pfrac4 + (R.kb.x + g));
-                const float4 p1 = __ldg(k.pfrac4 + (R.kb.y + g));
-                const float pfrac = dot4(R.wpl0, p0) + dot4(R.wpl1, p1);
+                const LwRec& R = recs[slot * CL + i];
+                GasRows r;
+                const int a = (upper >> i) & 1;
+                const MinorRef mr = a ? mr1 : mr0;
+                load_rows<false>(gas_tab(k), R.kb, g, mr.nmax, r);
+                const float tau = tau_abs<false, DENSE>(gas_tab(k), R, a, g, r, mr, &sm_sc4[jl * k.max_nscal].x, 4) +
+                                  R.aux.w;
+                const float pfrac = planck_fraction(R, r);
                 vtau[i] = tau;
                 vpf[i] = pfrac;
                 lw_layer_terms(tau, D, pfrac * R.aux.x, pfrac * R.aux.z, pfrac * R.aux.y, omt[i], sdn[i], sup[i]);
                 if (j == nlay - 1) {
-                    for (int rr = 0; rr < CS; ++rr) at_rank(sm_sfc, rr)[lane] = pfrac * R.aux2;
+                    for (int rr = 0; rr < CS; ++rr) at_rank(sm_sfc, rr)[lane] = pfrac * R.mix.w;
                     pf_bottom = pfrac;
                 }
             } else if (j == nlay - 1) {
@@ -428,13 +431,13 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
             ib = (1.f - omt[i]) * ib + b_here + hj * omt[i];
             gT[i] = 0.f; gH[i] = 0.f; gO[i] = 0.f; gS[i] = 0.f;
             if (j < nlay && gv) {
-                const Rec& R = recs[slot * CL + i];
+                const LwRec& R = recs[slot * CL + i];
                 const DRec& DR = drecs[slot * CL + i];
                 // table corners first: their latency overlaps the layer terms below
-                const float4 c0 = __ldg(k.kmaj4 + (R.kb.x + g));
-                const float4 c1 = __ldg(k.kmaj4 + (R.kb.y + g));
-                const float4 p0 = __ldg(k.pfrac4 + (R.kb.x + g));
-                const float4 p1 = __ldg(k.pfrac4 + (R.kb.y + g));
+                GasRows r;
+                const int a = (upper >> i) & 1;
+                const MinorRef mr = a ? mr1 : mr0;
+                load_rows<false>(gas_tab(k), R.kb, g, mr.nmax, r);
                 const float pf = vpf[i];
                 const float lay = pf * R.aux.x, ldn = pf * R.aux.z, lup = pf * R.aux.y;
                 float om, fact, domt, dfact;
@@ -450,15 +453,14 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
                 gL[i] += lupb * pf * DR.dB.y;       // level above layer i
                 gL[i + 1] += ldnb * pf * DR.dB.z;   // level below layer i
                 if (j == nlay - 1) {
-                    pfb += Sbar * R.aux2;
+                    pfb += Sbar * R.mix.w;
                     gTs += Sbar * pf_bottom * DR.dB.w;
                 }
                 float gh = 0.f, go = 0.f;
-                tau_abs_adjoint<DENSE>(k, R, DR, g, R.a ? mg1 : mg0, R.a ? nm1 : nm0, tb, c0, c1, sm_sc4 + jl * k.max_nscal,
-                                gt, gh, go);
-                gt += pfb * (dot4(DR.pT0, p0) + dot4(DR.pT1, p1));
-                gh += pfb * (dot4(DR.pH0, p0) + dot4(DR.pH1, p1));
-                go += pfb * (dot4(DR.pO0, p0) + dot4(DR.pO1, p1));
+                tau_abs_adjoint<false, DENSE>(gas_tab(k), R, DR, a, g, r, mr, tb, sm_sc4 + jl * k.max_nscal, gt, gh, go);
+                gt += pfb * (dot4(DR.pT0, r.p0) + dot4(DR.pT1, r.p1));
+                gh += pfb * (dot4(DR.pH0, r.p0) + dot4(DR.pH1, r.p1));
+                go += pfb * (dot4(DR.pO0, r.p0) + dot4(DR.pO1, r.p1));
                 gT[i] = gt;
                 gH[i] = gh;
                 gO[i] = go;

@@ -64,13 +64,6 @@ struct SwAdjOut {
 
 using D4 = Dual<4>;
 
-// Minor-interval code n < 3 (contributor << kScalBits | scaling kind) of a g-point's list
-// (minor_entry); codes 4, 5, ... come from gx = minor_gx[a] + g * minor_gx_stride.
-__device__ __forceinline__ int minor_code(const int4& mg, int n)
-{
-    return n == 0 ? mg.y : (n == 1 ? mg.z : mg.w);
-}
-
 // Adjoint of one (layer, g-point) from the adjoints of its two-stream outputs (R, T, Rdir,
 // Tdir, Tn, adif, adir) to the optical inputs of the layer: gas absorption tau (x), Rayleigh
 // tau (y), cloud tau (z), cloud tau*ssa (w) and cloud tau*ssa*g (v).  The combination is
@@ -346,60 +339,20 @@ struct LayerAdj {
 };
 
 template <bool DENSE>
-__device__ __noinline__ LayerAdj sw_layer_adjoint(const float4* __restrict__ kmaj4, const float2* __restrict__ kmin,
-                                                  const float2* __restrict__ krayl2, const Rec* Rc, const DRec* DR,
-                                                  const float4* sc4, const int* gx, int g, int4 mg, int nmax,
-                                                  float tau, float w0, float omw, float gasy, float mu0, float mu0_inv,
-                                                  float Rb, float Tb, float Rdb, float Tdb, float Tnb, float Afb,
-                                                  float Arb)
+__device__ __noinline__ LayerAdj sw_layer_adjoint(const GasTab kt, const SwRec* Rc, const DRec* DR, const float4* sc4,
+                                                  int a, int g, const MinorRef mr, float tau, float w0, float omw,
+                                                  float gasy, float mu0, float mu0_inv, float Rb, float Tb, float Rdb,
+                                                  float Tdb, float Tnb, float Afb, float Arb)
 {
-    const float4 c0 = __ldg(kmaj4 + (Rc->kb.x + g));
-    const float4 c1 = __ldg(kmaj4 + (Rc->kb.y + g));
-    float4 cr[3];
-#pragma unroll
-    for (int n = 0; n < 3; ++n) {
-        cr[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < nmax) {
-            const int c = minor_code(mg, n) >> kScalBits;
-            const float2 lo = __ldg(kmin + (Rc->kb.z + c));
-            const float2 hi = __ldg(kmin + (Rc->kb.w + c));
-            cr[n] = make_float4(lo.x, lo.y, hi.x, hi.y);
-        }
-    }
-    const float2 r0 = __ldg(krayl2 + (Rc->kr[0] + g));
-    const float2 r1 = __ldg(krayl2 + (Rc->kr[1] + g));
+    GasRows rows;
+    load_rows<true>(kt, Rc->kb, g, mr.nmax, rows);
 
     const LocalAdj la = sw_local_adjoint(tau, w0, omw, gasy, mu0, mu0_inv, Rb, Tb, Rdb, Tdb, Tnb, Afb, Arb);
 
-    float dT = dot4(DR->wT0, c0) + dot4(DR->wT1, c1);
-    float dH = dot4(DR->wH0, c0) + dot4(DR->wH1, c1);
-    float dO = dot4(DR->wO0, c0) + dot4(DR->wO1, c1);
-    auto minor_term = [&](int code, const float4& crn, bool on) {
-        const float M = dot4(Rc->fm, crn);
-        const float4 S = sc4[code & (kMaxScal - 1)];   // scaling, d ln / dT, d / d h2o, d / d o3
-        const float tT = S.x * (S.y * M + dot4(DR->fmT, crn));
-        const float tH = S.z * M + S.x * dot4(DR->fmH, crn);
-        const float tO = S.w * M + S.x * dot4(DR->fmO, crn);
-        dT += on ? tT : 0.f;
-        dH += on ? tH : 0.f;
-        dO += on ? tO : 0.f;
-    };
-#pragma unroll
-    for (int n = 0; n < 3; ++n)
-        if (n < nmax) minor_term(minor_code(mg, n), cr[n], n < mg.x);
-    if constexpr (DENSE) {   // more than three intervals over some g-point
-        for (int n = 3; n < nmax; ++n) {
-            const int code = n < mg.x ? gx[n - 3] : mg.y;
-            const int c = code >> kScalBits;
-            const float2 lo = __ldg(kmin + (Rc->kb.z + c));
-            const float2 hi = __ldg(kmin + (Rc->kb.w + c));
-            minor_term(code, make_float4(lo.x, lo.y, hi.x, hi.y), n < mg.x);
-        }
-    }
-    const float tab = la.ta, trb = la.tr;
-    LayerAdj r{tab * dT, tab * dH, tab * dO, la.tc, la.tsc, la.tsg};
-    const float4 kr = make_float4(r0.x, r0.y, r1.x, r1.y);
-    const float colr = Rc->aux.x;
+    LayerAdj r{0.f, 0.f, 0.f, la.tc, la.tsc, la.tsg};
+    tau_abs_adjoint<true, DENSE>(kt, *Rc, *DR, a, g, rows, mr, la.ta, sc4, r.t, r.h, r.o);
+    const float4 kr = rayleigh_corners(rows);
+    const float colr = Rc->aux.x, trb = la.tr;
     r.t += trb * colr * dot4(DR->fmT, kr);
     r.h += trb * (colr * dot4(DR->fmH, kr) + DR->dB.x * dot4(Rc->fm, kr));
     r.o += trb * colr * dot4(DR->fmO, kr);
@@ -411,30 +364,14 @@ __device__ __noinline__ LayerAdj sw_layer_adjoint(const float4* __restrict__ kma
 struct LayerFwd { float tau, w0, omw, gasy, R, T, Rdir, Tdir, Tn, adif, adir; };
 
 template <bool DENSE>
-__device__ __noinline__ LayerFwd sw_layer_forward(const float4* __restrict__ kmaj4, const float2* __restrict__ kmin,
-                                                  const float2* __restrict__ krayl2, const Rec* Rc, const float4* sc4,
-                                                  const int* gx, int g, int4 mg, int nmax, float mu0, float mu0_inv)
+__device__ __noinline__ LayerFwd sw_layer_forward(const GasTab kt, const SwRec* Rc, const float4* sc4, int a, int g,
+                                                  const MinorRef mr, float mu0, float mu0_inv)
 {
-    const float4 c0 = __ldg(kmaj4 + (Rc->kb.x + g));
-    const float4 c1 = __ldg(kmaj4 + (Rc->kb.y + g));
-    float ta = dot4(Rc->wmaj0, c0) + dot4(Rc->wmaj1, c1);
-    auto minor_term = [&](int code, bool on) {
-        const int c = code >> kScalBits;
-        const float2 lo = __ldg(kmin + (Rc->kb.z + c));
-        const float2 hi = __ldg(kmin + (Rc->kb.w + c));
-        const float t = sc4[code & (kMaxScal - 1)].x *
-                        (Rc->fm.x * lo.x + Rc->fm.y * lo.y + Rc->fm.z * hi.x + Rc->fm.w * hi.y);
-        ta += on ? t : 0.f;
-    };
-#pragma unroll
-    for (int n = 0; n < 3; ++n)
-        if (n < nmax) minor_term(minor_code(mg, n), n < mg.x);
-    if constexpr (DENSE)
-        for (int n = 3; n < nmax; ++n) minor_term(n < mg.x ? gx[n - 3] : mg.y, n < mg.x);
+    GasRows rows;
+    load_rows<true>(kt, Rc->kb, g, mr.nmax, rows);
+    const float ta = tau_abs<true, DENSE>(kt, *Rc, a, g, rows, mr, &sc4->x, 4);
+    const float tr = dot4(Rc->fm, rayleigh_corners(rows)) * Rc->aux.x;
     LayerFwd o;
-    const float2 r0 = __ldg(krayl2 + (Rc->kr[0] + g));
-    const float2 r1 = __ldg(krayl2 + (Rc->kr[1] + g));
-    const float tr = (Rc->fm.x * r0.x + Rc->fm.y * r0.y + Rc->fm.z * r1.x + Rc->fm.w * r1.y) * Rc->aux.x;
     o.tau = ta + tr + Rc->aux.y;
     const float ts = tr + Rc->aux.z;
     o.w0 = 0.f;
@@ -525,7 +462,7 @@ __host__ __device__ __forceinline__ SwAdjLayout sw_adj_layout(int ngas, int nban
     L.x4 = align16(L.x3 + sizeof(float2) * nw);
     L.x5 = align16(L.x4 + (sizeof(float4) + sizeof(float)) * nw);
     L.recs = align16(L.x5 + sizeof(float2) * nw);
-    L.drecs = align16(L.recs + sizeof(Rec) * size_t(kLPC) * mgb * nbuf);
+    L.drecs = align16(L.recs + sizeof(SwRec) * size_t(kLPC) * mgb * nbuf);
     L.total = align16(L.drecs + sizeof(DRec) * size_t(kLPC) * mgb * nbuf);
     return L;
 }
@@ -579,7 +516,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
     float4* sm_x4a = reinterpret_cast<float4*>(smem_raw + SL.x4);
     float* sm_x4b = reinterpret_cast<float*>(sm_x4a + NWt * 32);
     float2* sm_x5 = reinterpret_cast<float2*>(smem_raw + SL.x5);
-    Rec* const recs0 = reinterpret_cast<Rec*>(smem_raw + SL.recs) + w * CL * mgb;
+    SwRec* const recs0 = reinterpret_cast<SwRec*>(smem_raw + SL.recs) + w * CL * mgb;
     DRec* const drecs0 = reinterpret_cast<DRec*>(smem_raw + SL.drecs) + w * CL * mgb;
 
     const bool top_at_1 = play[icol] < play[icol + size_t(nlay - 1) * ncol];
@@ -637,6 +574,10 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
     }
     __syncthreads();
 
+    // bit i: layer i of this warp's chunk is in the upper atmosphere
+    const unsigned upper = __ballot_sync(0xffffffffu, lane < CL && j0 + w * CL + lane < nlay &&
+                                                          st[w * CL + (lane < CL ? lane : 0)].itropo);
+
     const int ngpt = k.ngpt;
     // top / bottom boundary seeds (every thread walks the whole column)
     const float al0 = seed_at(seed_up, 0);
@@ -655,10 +596,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
         const int b0 = k.group_band0[gg];
         const int gband = gv ? k.gpt2band[g] : b0;
         const int slot = gband - b0;
-        const int4 mg0 = minor_entry(k.minor_g[0], g, gv);
-        const int4 mg1 = minor_entry(k.minor_g[1], g, gv);
-        const int nm0 = __reduce_max_sync(0xffffffffu, mg0.x);
-        const int nm1 = __reduce_max_sync(0xffffffffu, mg1.x);
+        const MinorRef mr0 = minor_ref(k, 0, g, gv), mr1 = minor_ref(k, 1, g, gv);
         const float ad = gv ? __ldg(alb_dir + gband + size_t(icol) * nband) : 0.f;
         const float af = gv ? __ldg(alb_dif + gband + size_t(icol) * nband) : 0.f;
 
@@ -666,7 +604,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
         // records of groups gg and gg + 1 are built together at even gg into two buffers: with
         // 8 layers and 2 bands a group has 16 records per warp, so one group alone leaves half
         // the lanes idle.
-        Rec* const recs = recs0 + (PAIR ? (gg & 1) : 0) * kLPC * mgb;
+        SwRec* const recs = recs0 + (PAIR ? (gg & 1) : 0) * kLPC * mgb;
         DRec* const drecs = drecs0 + (PAIR ? (gg & 1) : 0) * kLPC * mgb;
         if (!PAIR || (gg & 1) == 0) {
             const int nrec = CL * mgb;
@@ -705,10 +643,10 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             float R = 0.f, T = 1.f, Rdir = 0.f, Tdir = 0.f, Tn = 1.f, adif = 0.f, adir = 0.f;
             float tau = 0.f, w0 = 0.f, omw = 1.f, gasy = 0.f;
             if (j < nlay && gv) {
-                const Rec& Rc = recs[slot * CL + i];
-                const LayerFwd lf = sw_layer_forward<DENSE>(k.kmaj4, k.kmin2[Rc.a], k.krayl2, &Rc, sm_sc4 + jl * k.max_nscal,
-                                                     k.minor_gx[Rc.a] + size_t(g) * k.minor_gx_stride, g,
-                                                     Rc.a ? mg1 : mg0, Rc.a ? nm1 : nm0, mu0, mu0_inv);
+                const SwRec& Rc = recs[slot * CL + i];
+                const int a = (upper >> i) & 1;
+                const LayerFwd lf = sw_layer_forward<DENSE>(gas_tab(k), &Rc, sm_sc4 + jl * k.max_nscal, a, g,
+                                                            a ? mr1 : mr0, mu0, mu0_inv);
                 tau = lf.tau; w0 = lf.w0; omw = lf.omw; gasy = lf.gasy;
                 R = lf.R; T = lf.T; Rdir = lf.Rdir; Tdir = lf.Tdir; Tn = lf.Tn; adif = lf.adif; adir = lf.adir;
             }
@@ -969,12 +907,11 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             Db = sm_be[jl] + sm_ga[jl] + sm_hh[jl] * vAr[i] + vSub[i] * vRd[i] + vSdb[i] * vTd[i] + vTn[i] * Db;
             gT[i] = 0.f; gH[i] = 0.f; gO[i] = 0.f; gC0[i] = 0.f; gC1[i] = 0.f; gC2[i] = 0.f;
             if (j < nlay && gv) {
-                const Rec& Rc = recs[slot * CL + i];
-                const LayerAdj la = sw_layer_adjoint<DENSE>(k.kmaj4, k.kmin2[Rc.a], k.krayl2, &Rc, &drecs[slot * CL + i],
-                                                     sm_sc4 + jl * k.max_nscal,
-                                                     k.minor_gx[Rc.a] + size_t(g) * k.minor_gx_stride, g,
-                                                     Rc.a ? mg1 : mg0, Rc.a ? nm1 : nm0, vTau[i], vW0[i], vOmw[i],
-                                                     vG[i], mu0, mu0_inv, vRb[i], vTb[i], Rdb, Tdb, Tnb, vAfb[i], Arb);
+                const SwRec& Rc = recs[slot * CL + i];
+                const int a = (upper >> i) & 1;
+                const LayerAdj la = sw_layer_adjoint<DENSE>(
+                    gas_tab(k), &Rc, &drecs[slot * CL + i], sm_sc4 + jl * k.max_nscal, a, g, a ? mr1 : mr0, vTau[i],
+                    vW0[i], vOmw[i], vG[i], mu0, mu0_inv, vRb[i], vTb[i], Rdb, Tdb, Tnb, vAfb[i], Arb);
                 gT[i] = la.t; gH[i] = la.h; gO[i] = la.o;
                 gC0[i] = la.tc; gC1[i] = la.tsc; gC2[i] = la.tsg;
             }

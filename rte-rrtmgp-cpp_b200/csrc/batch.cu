@@ -264,9 +264,10 @@ size_t team_smem_bytes(const rrtmgp_b200_batch_t* b, int domain, int nlay, int c
     const KdistView<float>& v = b->k[domain]->v32;
     const int W = ceil_div_i(nlay, cl);
     // as the column code lays it out: by capacity, W cl layers
-    const SmemLayout L = domain == 0 ? smem_layout(W * cl, v.ngas, v.nband, 1, W, 2, cl, v.max_group_bands, v.max_nscal)
+    const SmemLayout L = domain == 0 ? smem_layout(W * cl, v.ngas, v.nband, 1, W, 2, cl, v.max_group_bands, v.max_nscal,
+                                                   sizeof(LwRec))
                                      : smem_layout(W * cl, v.ngas, v.nband, 0, W, 3, cl,
-                                                   v.max_group_bands * (cl == 8 ? 2 : 1), v.max_nscal);
+                                                   v.max_group_bands * (cl == 8 ? 2 : 1), v.max_nscal, sizeof(SwRec));
     return align16(L.total);
 }
 

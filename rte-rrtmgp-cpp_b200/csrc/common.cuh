@@ -68,6 +68,11 @@ constexpr int kMaxGases = 24;          // gases in one k-distribution after redu
 constexpr int kMaxBandGpt = 32;        // g-points per band handled in registers/shared mem
 constexpr int kMaxBands = 64;
 
+// Eight table values of one g-point, read with one 256-bit load (fused_common.cuh: ldg8).
+struct __align__(32) Tab8 {
+    float4 a, b;
+};
+
 // ---------------------------------------------------------------------------------------
 // Device-resident k-distribution in one precision.  All tables are g-point fastest so that
 // the g-points of a band at one (T, p, eta) corner are contiguous.
@@ -109,8 +114,13 @@ struct KdistView {
     int max_group_bands;            // most bands touched by one group
     int max_band_minor;             // most minor intervals in one (band, atmosphere)
     const int* group_band0;         // [ngroups] first band of each group
-    // Corner-packed copies for the fused FP32 kernels (NULL in the FP64 view):
+    // Corner-packed copies for the FP32 kernels (NULL in the FP64 view):
     //   kmaj4/pfrac4 [t][p][eta][g], p < npres, eta < neta-1: (k(e,p), k(e+1,p), k(e,p+1), k(e+1,p+1))
+    //   kmp8         [t][p][eta][g] (longwave, fused kernels): a = kmaj4, b = pfrac4, so that one
+    //                256-bit load returns both (8192 x 128 forward 3.03 ms, 3.25 with two
+    //                128-bit loads); the per-stage kernel is faster on the separate tables (0.63
+    //                and 0.66 ms at 4096 x 91).
+    // Per-stage kernels (lanes = columns, one g-point at a time):
     //   kmin2[a]     [t][eta][c], eta < neta-1: (k(e), k(e+1))
     //   krayl2       [a][t][eta][g], eta < neta-1: (k(e), k(e+1))
     //   minor_g[a]   [g]: x = number of intervals covering g, y/z/w = the first three codes
@@ -118,13 +128,25 @@ struct KdistView {
     //                interval (below); unused slots repeat y (0 when no interval covers g).
     //   minor_gx[a]  [g][minor_gx_stride]: codes 4, 5, ... of g (NULL when no g-point has
     //                more than three intervals).
+    // Fused kernels (lanes = the g-points of a group of 32): the minor-interval coefficients by
+    // g-point, in aligned rows that a warp reads with one load per row,
+    //   kmin4        [a][t][eta][u][g]: two (k(e), k(e+1)) pairs; the pairs of g are, in this
+    //                order, the Rayleigh coefficient's (shortwave only) and those of its minor
+    //                intervals in their file order, zero past the last
+    //   minor_s      [a][u][g]: x = scaling kinds (below) of the unit's two pairs, one byte each;
+    //                y = minor intervals of g
+    // (units u < nminor_units).
     const float4* kmaj4;
     const float4* pfrac4;
+    const Tab8* kmp8;
     const float2* kmin2[2];
     const float2* krayl2;
     const int4* minor_g[2];
     const int* minor_gx[2];
     int minor_gx_stride;
+    const float4* kmin4;
+    const int2* minor_s;
+    int nminor_units;
     int max_minor_per_g;            // most intervals covering one g-point
     // Scaling kinds: intervals whose scaling (gas_optical_depths_minor_kernel,
     // gas_optics_rrtmgp_kernels.cu:396-417) is the same function of the layer -- same minor
@@ -139,7 +161,7 @@ struct KdistView {
 };
 
 constexpr int kScalBits = 6;                    // bits of a scaling kind in a minor code
-constexpr int kMaxScal = 1 << kScalBits;        // scaling kinds per atmosphere (fused kernels)
+constexpr int kMaxScal = 1 << kScalBits;        // scaling kinds per atmosphere (minor codes, minor_s bytes)
 
 }  // namespace rrtmgp_b200
 

@@ -34,7 +34,7 @@ int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     const int CS = (NW + 15) / 16, NWc = (NW + CS - 1) / CS;
     RB_CHECK_ARG(CS <= 8, "forward_lw: nlay too large for the fused kernel (at most 128 chunks)");
     const size_t smem = smem_layout(NWc * CL, v.ngas, v.nband, 1, CS * NWc, 2, CL,
-                                    v.max_group_bands * (CL == 8 ? 2 : 1), v.max_nscal, NWc).total;
+                                    v.max_group_bands * (CL == 8 ? 2 : 1), v.max_nscal, sizeof(LwRec), NWc).total;
     if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_lw: shared memory need exceeds 220 KB");
     static PerDeviceOnce attr;
     int st = attr.run([] {

@@ -35,7 +35,7 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     const int CS = (NW + 15) / 16, NWc = (NW + CS - 1) / CS;
     RB_CHECK_ARG(CS <= 8, "forward_sw: nlay too large for the fused kernel (at most 128 chunks)");
     const size_t smem = smem_layout(NWc * CL, v.ngas, v.nband, aer.present ? 4 : 0, CS * NWc, 3, CL,
-                                    v.max_group_bands * (CL == 8 ? 2 : 1), v.max_nscal, NWc).total;
+                                    v.max_group_bands * (CL == 8 ? 2 : 1), v.max_nscal, sizeof(SwRec), NWc).total;
     if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_sw: shared memory need exceeds 220 KB");
     static PerDeviceOnce attr;
     int st = attr.run([] {

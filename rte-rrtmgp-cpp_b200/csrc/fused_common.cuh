@@ -27,23 +27,33 @@ struct __align__(16) LayerState {
     float t_top, t_bot, dp, pad2;
 };
 
-// Per (layer, band) record.
-struct __align__(16) Rec {
-    int4 kb;          // x, y: element offsets (row * ngpt) of the kmaj4/pfrac4 rows of
-                      //       (t0, p0, e0) and (t1, p0, e1); z, w: kmin2 row offsets of (t0, e0), (t1, e1)
-    float4 wmaj0, wmaj1;   // col_mix x fmajor (major absorption weights)
-    float4 wpl0, wpl1;     // fmajor (Planck fractions; SW: unused)
-    float4 fm;             // fminor (minor and Rayleigh weights)
-    float4 aux;            // LW: pl_lay, pl_top, pl_bot, tau_cloud
-                           // SW: col_dry + col_h2o (Rayleigh), cloud tau, ssa, g
-    float aux2;            // LW: surface Planck function (bottom layer only)
-                           // SW: cloud absorption optical depth tau_c * (1 - ssa_c)
-    int a;                 // 0 lower / 1 upper atmosphere
-    int kr[2];             // element offsets (row * ngpt) of the krayl2 rows of (a, t0, e0), (a, t1, e1)
-    int4 pad;              // 144 bytes: an odd number of 16-byte units, so that the 128-bit stores of
-                           // 32 lanes building consecutive records spread over all 32 banks
+// Per (layer, band) records.  Their sizes are odd numbers of 16-byte units, so that the 128-bit
+// stores of 32 lanes building consecutive records spread over all 32 banks.
+//
+// Longwave: only what the weights cannot be formed from (the major and the Planck weights are
+// products of fm, fpress and col_mix, a dozen multiplies per lane of a kernel whose FMA pipe is a
+// quarter used), because shared memory held by records is taken from the L1 that holds the
+// table rows: with 144-byte records a third of the table sectors missed it.
+struct __align__(16) LwRec {
+    int4 kb;          // x, y: element offsets (row * ngpt) of the kmp8 rows of (t0, p0, e0) and
+                      //       (t1, p0, e1); z, w: kmin4 rows of (a, t0, e0), (a, t1, e1), unit 0
+    float4 fm;        // fminor (minor weights)
+    float4 mix;       // col_mix at the two temperatures, fpress, surface Planck function (bottom layer only)
+    float4 aux;       // pl_lay, pl_top, pl_bot, tau_cloud
+    int4 pad;
 };
-static_assert(sizeof(Rec) == 144, "Rec stride");
+static_assert(sizeof(LwRec) == 80, "LwRec stride");
+
+// Shortwave: the kernel is bound by instruction issue, so the weights are stored as they are used.
+struct __align__(16) SwRec {
+    int4 kb;               // as LwRec, on the kmaj4 rows
+    float4 wmaj0, wmaj1;   // col_mix x fmajor (major absorption weights)
+    float4 fm;             // fminor (minor and Rayleigh weights)
+    float4 aux;            // col_dry + col_h2o (Rayleigh), cloud tau, tau*ssa, tau*ssa*g
+    float aux2;            // cloud absorption optical depth tau_c * (1 - ssa_c)
+    int pad[7];
+};
+static_assert(sizeof(SwRec) == 112, "SwRec stride");
 
 // Reduce-scatter of N per-lane values over 32 lanes: afterwards lane L holds in v[0] the warp
 // total of value L >> log2(32 / N) (N <= 32, a power of two).
@@ -82,11 +92,11 @@ __device__ __forceinline__ float warp_sum(float x)
     return x;
 }
 
-// Interpolation part of a record (interpolation_kernel, gas_optics_rrtmgp_kernels.cu:256-291)
-// for band b at layer state s.  The minor scalings are per layer, not per record
-// (layer_minor_scalings).
-__device__ __forceinline__ void record_weights(const KdistView<float>& k, Rec& R, const LayerState& s,
-                                               const float* cg, int cgs, int b)
+// Interpolation of band b at layer state s (interpolation_kernel,
+// gas_optics_rrtmgp_kernels.cu:256-291): its weights, and the table rows of a record.  The minor
+// scalings are per layer, not per record (layer_minor_scalings).
+__device__ __forceinline__ FlavorWeights<float> record_rows(const KdistView<float>& k, int4& kb, const LayerState& s,
+                                                            const float* cg, int cgs, int b)
 {
     LayerInterp<float> li;
     li.jt = s.jt;
@@ -94,26 +104,36 @@ __device__ __forceinline__ void record_weights(const KdistView<float>& k, Rec& R
     li.itropo = s.itropo;
     li.ftemp = s.ftemp;
     li.fpress = s.fpress;
-    const int flav = k.band_flav[2 * b + li.itropo];
-    const FlavorWeights<float> fw = flavor_weights(k, flav, li, cg, cgs);
-    const int ne1 = k.neta - 1, np = k.npres;
-    const int p0 = li.jp + li.itropo - 1;
-    R.kb.x = (((li.jt - 1) * np + p0) * ne1 + (fw.j0 - 1)) * k.ngpt;
-    R.kb.y = ((li.jt * np + p0) * ne1 + (fw.j1 - 1)) * k.ngpt;
     const int a = li.itropo;
-    const int nc = k.ncontrib[a] > 0 ? k.ncontrib[a] : 1;
-    // kmin2 rows; the Rayleigh rows (krayl2, [a][t][eta][g]) follow the same (t, eta) corners.
-    R.kb.z = ((li.jt - 1) * ne1 + (fw.j0 - 1)) * nc;
-    R.kb.w = (li.jt * ne1 + (fw.j1 - 1)) * nc;
-    const float fp = li.fpress, f1 = 1.f - li.fpress;
-    R.wpl0 = make_float4(f1 * fw.fm[0], f1 * fw.fm[1], fp * fw.fm[0], fp * fw.fm[1]);
-    R.wpl1 = make_float4(f1 * fw.fm[2], f1 * fw.fm[3], fp * fw.fm[2], fp * fw.fm[3]);
-    R.wmaj0 = make_float4(fw.cm[0] * R.wpl0.x, fw.cm[0] * R.wpl0.y, fw.cm[0] * R.wpl0.z, fw.cm[0] * R.wpl0.w);
-    R.wmaj1 = make_float4(fw.cm[1] * R.wpl1.x, fw.cm[1] * R.wpl1.y, fw.cm[1] * R.wpl1.z, fw.cm[1] * R.wpl1.w);
+    const FlavorWeights<float> fw = flavor_weights(k, k.band_flav[2 * b + a], li, cg, cgs);
+    const int ne1 = k.neta - 1, np = k.npres;
+    const int p0 = li.jp + a - 1;
+    const int mrow = k.nminor_units * k.ngpt;
+    kb = make_int4((((li.jt - 1) * np + p0) * ne1 + (fw.j0 - 1)) * k.ngpt,
+                   ((li.jt * np + p0) * ne1 + (fw.j1 - 1)) * k.ngpt,
+                   ((a * k.ntemp + li.jt - 1) * ne1 + (fw.j0 - 1)) * mrow,
+                   ((a * k.ntemp + li.jt) * ne1 + (fw.j1 - 1)) * mrow);
+    return fw;
+}
+
+__device__ __forceinline__ void record_weights(const KdistView<float>& k, LwRec& R, const LayerState& s,
+                                               const float* cg, int cgs, int b, float planck_sfc)
+{
+    const FlavorWeights<float> fw = record_rows(k, R.kb, s, cg, cgs, b);
     R.fm = make_float4(fw.fm[0], fw.fm[1], fw.fm[2], fw.fm[3]);
-    R.a = a;
-    R.kr[0] = ((a * k.ntemp + li.jt - 1) * ne1 + (fw.j0 - 1)) * k.ngpt;
-    R.kr[1] = ((a * k.ntemp + li.jt) * ne1 + (fw.j1 - 1)) * k.ngpt;
+    R.mix = make_float4(fw.cm[0], fw.cm[1], s.fpress, planck_sfc);
+}
+
+__device__ __forceinline__ void record_weights(const KdistView<float>& k, SwRec& R, const LayerState& s,
+                                               const float* cg, int cgs, int b)
+{
+    const FlavorWeights<float> fw = record_rows(k, R.kb, s, cg, cgs, b);
+    R.fm = make_float4(fw.fm[0], fw.fm[1], fw.fm[2], fw.fm[3]);
+    const float fp = s.fpress, f1 = 1.f - s.fpress;
+    R.wmaj0 = make_float4(fw.cm[0] * (f1 * fw.fm[0]), fw.cm[0] * (f1 * fw.fm[1]), fw.cm[0] * (fp * fw.fm[0]),
+                          fw.cm[0] * (fp * fw.fm[1]));
+    R.wmaj1 = make_float4(fw.cm[1] * (f1 * fw.fm[2]), fw.cm[1] * (f1 * fw.fm[3]), fw.cm[1] * (fp * fw.fm[2]),
+                          fw.cm[1] * (fp * fw.fm[3]));
 }
 
 // Minor scaling of scaling kind sid of atmosphere a at a layer (minor_scaling: the same
@@ -150,65 +170,151 @@ __device__ __forceinline__ void layer_minor_scalings(const KdistView<float>& k, 
     }
 }
 
-// Code n of g-point g's minor-interval list (minor_g / minor_gx; n < count, or a code that
-// repeats the first one for n < 3).
-__device__ __forceinline__ int minor_code_at(const KdistView<float>& k, int a, const int4& mg, int g, int n)
+// One 256-bit load of a table row entry (sm_100; p is 32-byte aligned: Tab8).
+__device__ __forceinline__ Tab8 ldg8(const Tab8* p)
 {
-    if (n < 3) return n == 0 ? mg.y : (n == 1 ? mg.z : mg.w);
-    return n < mg.x ? __ldg(k.minor_gx[a] + size_t(g) * k.minor_gx_stride + (n - 3)) : mg.y;
+    Tab8 r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+        : "l"(p));
+    return r;
 }
 
-// Absorption optical depth of g-point g from a record: major (8 corners via two float4 loads)
-// plus the minor intervals covering g (minor_g list), as gas_optical_depths_major/minor.
-// nmax = most intervals over the warp's lanes (warp-uniform loop bound); lanes with fewer
-// intervals read a valid entry and discard it with a select, so the loop does not diverge.
-// sc: the layer's scalings, kind sid at sc[sid * sst].  DENSE: tables with more than three
-// intervals over some g-point (KdistView::max_minor_per_g > 3); the loop over the further
-// intervals is compiled only then, so that for the usual layouts the whole function stays
-// straight-line code whose table loads the caller's unrolled layer loop can overlap.
-template <bool DENSE = false>
-__device__ __forceinline__ float tau_abs(const KdistView<float>& k, const Rec& R, int g, int4 mg, int nmax,
-                                         const float* sc, int sst = 1)
+// 128-bit load when on, else zeros: one predicated load instead of a branch around it, so that the
+// loads of several unrolled layers can be in flight together.  (Without the zeros the
+// registers of an unrolled loop's loads are live from its start: 2 KB of spills.)
+__device__ __forceinline__ float4 ldg4_if(const float4* p, bool on)
 {
-    const float4 c0 = __ldg(k.kmaj4 + (R.kb.x + g));
-    const float4 c1 = __ldg(k.kmaj4 + (R.kb.y + g));
-    float tau = R.wmaj0.x * c0.x + R.wmaj0.y * c0.y + R.wmaj0.z * c0.z + R.wmaj0.w * c0.w +
-                R.wmaj1.x * c1.x + R.wmaj1.y * c1.y + R.wmaj1.z * c1.z + R.wmaj1.w * c1.w;
-    const float2* kn = k.kmin2[R.a];
-#pragma unroll
-    for (int n = 0; n < 3; ++n) {
-        if (n < nmax) {
-            const int code = n == 0 ? mg.y : (n == 1 ? mg.z : mg.w);
-            const int c = code >> kScalBits;
-            const float2 lo = __ldg(kn + (R.kb.z + c));
-            const float2 hi = __ldg(kn + (R.kb.w + c));
-            const float t = sc[(code & (kMaxScal - 1)) * sst] *
-                            (R.fm.x * lo.x + R.fm.y * lo.y + R.fm.z * hi.x + R.fm.w * hi.y);
-            tau += (n < mg.x) ? t : 0.f;
-        }
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+f"(r.x), "+f"(r.y), "+f"(r.z), "+f"(r.w)
+        : "l"(p), "r"(int(on)));
+    return r;
+}
+
+__device__ __forceinline__ float dot4(const float4& a, const float4& b)
+{
+    return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
+}
+
+// Sum over (eta, p) of one temperature's corners: f0, f1 the fminor weights of the two etas.
+__device__ __forceinline__ float corner_sum(float f0, float f1, float fp, const float4& c)
+{
+    return (1.f - fp) * (f0 * c.x + f1 * c.y) + fp * (f0 * c.z + f1 * c.w);
+}
+
+// The minor intervals of a lane's g-point in one atmosphere: the scaling kinds of the pairs of units
+// 0 and 1 (a byte each; 0 past the last interval) and the most intervals over the warp's lanes.
+struct MinorRef {
+    int sid0, sid1, nmax;
+};
+
+// The gas tables of one domain, by value for out-of-line callers.
+struct GasTab {
+    const float4* kmaj4;   // shortwave
+    const Tab8* kmp8;      // longwave
+    const float4* kmin4;
+    const int2* minor_s;
+    int ngpt, nunits;
+};
+__device__ __forceinline__ GasTab gas_tab(const KdistView<float>& k)
+{
+    return GasTab{k.kmaj4, k.kmp8, k.kmin4, k.minor_s, k.ngpt, k.nminor_units};
+}
+
+__device__ __forceinline__ MinorRef minor_ref(const KdistView<float>& k, int a, int g, bool valid)
+{
+    const int2* const m = k.minor_s + size_t(a) * k.nminor_units * k.ngpt + g;
+    const int2 e = valid ? __ldg(m) : make_int2(0, 0);
+    return MinorRef{e.x, valid && k.nminor_units > 1 ? __ldg(m + k.ngpt).x : 0, __reduce_max_sync(0xffffffffu, e.y)};
+}
+
+// The table values of one (layer, g-point): the two major corner rows, the longwave's
+// Planck-fraction rows, the minor rows of units 0 and 1 (shortwave: pair 0 of unit 0 is the
+// Rayleigh coefficient), zeros where no lane of the warp needs them.  Loaded together, before any
+// of them is used.
+struct GasRows {
+    float4 c0, c1;   // kmajor corners
+    float4 p0, p1;   // LW: Planck fraction corners
+    float4 m0, m1;   // minor rows, unit 0
+    float4 n0, n1;   // minor rows, unit 1
+};
+template <bool SW>
+__device__ __forceinline__ void load_rows(const GasTab& k, const int4& kb, int g, int nmax, GasRows& r)
+{
+    if constexpr (SW) {
+        r.c0 = __ldg(k.kmaj4 + (kb.x + g));
+        r.c1 = __ldg(k.kmaj4 + (kb.y + g));
+        r.m0 = __ldg(k.kmin4 + (kb.z + g));
+        r.m1 = __ldg(k.kmin4 + (kb.w + g));
+    } else {
+        const Tab8 t0 = ldg8(k.kmp8 + (kb.x + g)), t1 = ldg8(k.kmp8 + (kb.y + g));
+        r.c0 = t0.a; r.p0 = t0.b;
+        r.c1 = t1.a; r.p1 = t1.b;
+        r.m0 = ldg4_if(k.kmin4 + (kb.z + g), nmax > 0);
+        r.m1 = ldg4_if(k.kmin4 + (kb.w + g), nmax > 0);
     }
+    constexpr int n1 = SW ? 1 : 2;   // intervals in unit 0
+    r.n0 = ldg4_if(k.kmin4 + (kb.z + k.ngpt + g), nmax > n1);
+    r.n1 = ldg4_if(k.kmin4 + (kb.w + k.ngpt + g), nmax > n1);
+}
+
+// The (T, eta) corners in fminor order of the first and the second pair of two rows.
+__device__ __forceinline__ float4 pair0(const float4& x, const float4& y) { return make_float4(x.x, x.y, y.x, y.y); }
+__device__ __forceinline__ float4 pair1(const float4& x, const float4& y) { return make_float4(x.z, x.w, y.z, y.w); }
+__device__ __forceinline__ float4 rayleigh_corners(const GasRows& r) { return pair0(r.m0, r.m1); }
+
+// Visits the minor intervals of g-point g: f(corners in fminor order, scaling kind), in their file
+// order.  Lanes with fewer intervals than m.nmax (warp-uniform bound) take zero coefficients and
+// kind 0, so nothing diverges and no select is needed.  Units 0 and 1 come from r (load_rows).
+// DENSE: more than three intervals over some g-point (KdistView::max_minor_per_g > 3); the loop over
+// the further units is compiled only then.
+template <bool SW, bool DENSE, class F>
+__device__ __forceinline__ void for_minors(const GasTab& k, const int4& kb, int a, int g, const GasRows& r,
+                                           const MinorRef& m, F&& f)
+{
+    constexpr int R = SW ? 1 : 0;
+    if constexpr (!SW)
+        if (m.nmax > 0) f(pair0(r.m0, r.m1), m.sid0 & 255);
+    if (m.nmax > 1 - R) f(pair1(r.m0, r.m1), m.sid0 >> 8);
+    if (m.nmax > 2 - R) f(pair0(r.n0, r.n1), m.sid1 & 255);
+    if (m.nmax > 3 - R) f(pair1(r.n0, r.n1), m.sid1 >> 8);
     if constexpr (DENSE) {
-        for (int n = 3; n < nmax; ++n) {
-            const int code = minor_code_at(k, R.a, mg, g, n);
-            const int c = code >> kScalBits;
-            const float2 lo = __ldg(kn + (R.kb.z + c));
-            const float2 hi = __ldg(kn + (R.kb.w + c));
-            const float t = sc[(code & (kMaxScal - 1)) * sst] *
-                            (R.fm.x * lo.x + R.fm.y * lo.y + R.fm.z * hi.x + R.fm.w * hi.y);
-            tau += (n < mg.x) ? t : 0.f;
+        for (int u = 2; 2 * u - R < m.nmax; ++u) {
+            const int w = __ldg(&k.minor_s[(size_t(a) * k.nunits + u) * k.ngpt + g].x);
+            const float4 x0 = __ldg(k.kmin4 + (kb.z + u * k.ngpt + g));
+            const float4 x1 = __ldg(k.kmin4 + (kb.w + u * k.ngpt + g));
+            f(pair0(x0, x1), w & 255);
+            f(pair1(x0, x1), w >> 8);
         }
     }
+}
+
+// Absorption optical depth of g-point g from a record: major (8 corners) plus the minor
+// intervals covering g, as gas_optical_depths_major/minor.  r: load_rows of the record; the rest as
+// for_minors.  sc: the layer's scalings, kind sid at sc[sid * sst].
+__device__ __forceinline__ float major_tau(const LwRec& R, const GasRows& r)
+{
+    return R.mix.x * corner_sum(R.fm.x, R.fm.y, R.mix.z, r.c0) + R.mix.y * corner_sum(R.fm.z, R.fm.w, R.mix.z, r.c1);
+}
+__device__ __forceinline__ float major_tau(const SwRec& R, const GasRows& r)
+{
+    return dot4(R.wmaj0, r.c0) + dot4(R.wmaj1, r.c1);
+}
+template <bool SW, bool DENSE, class Rec>
+__device__ __forceinline__ float tau_abs(const GasTab& k, const Rec& R, int a, int g, const GasRows& r,
+                                         const MinorRef& m, const float* sc, int sst = 1)
+{
+    float tau = major_tau(R, r);
+    for_minors<SW, DENSE>(k, R.kb, a, g, r, m,
+                          [&](const float4& c, int sid) { tau += sc[sid * sst] * dot4(R.fm, c); });
     return tau;
 }
 
-// minor_g entry of g-point g with unused slots set to the first used one (or to contributor 0,
-// slot 0), so that tau_abs can read every slot below the warp's maximum count.
-__device__ __forceinline__ int4 minor_entry(const int4* mgt, int g, bool valid)
+// Planck fraction (Planck_source_kernel, gas_optics_rrtmgp_kernels.cu:181-190).
+__device__ __forceinline__ float planck_fraction(const LwRec& R, const GasRows& r)
 {
-    int4 m = valid ? __ldg(mgt + g) : make_int4(0, 0, 0, 0);
-    if (m.x < 2) m.z = m.y;
-    if (m.x < 3) m.w = m.y;
-    return m;
+    return corner_sum(R.fm.x, R.fm.y, R.mix.z, r.p0) + corner_sum(R.fm.z, R.fm.w, R.mix.z, r.p1);
 }
 
 // Context of a fused column computation.  Members: icol(); warp() = the chunk this warp owns
@@ -325,8 +431,8 @@ __device__ __forceinline__ void setup_layers(const KdistView<float>& k, const Ga
 // band or per g-point is accepted.
 inline bool fused_layout_ok(const KdistView<float>& v, bool sw, int max_bands)
 {
-    return v.kmaj4 && v.minor_in_band && v.nscal[0] <= kMaxScal && v.nscal[1] <= kMaxScal &&
-           v.max_group_bands <= max_bands && (sw ? v.krayl2 != nullptr : v.pfrac4 != nullptr);
+    return v.minor_in_band && v.nscal[0] <= kMaxScal && v.nscal[1] <= kMaxScal &&
+           v.max_group_bands <= max_bands && v.is_lw == !sw;
 }
 
 // Shared-memory offsets (bytes) of the fused kernels, all 16-byte aligned.
@@ -337,10 +443,10 @@ struct SmemLayout {
 __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
 // nlay: layers whose state the CTA holds; NW: chunks of the column (maps); NWloc: warps of
-// the CTA (records).
+// the CTA (records of rec_bytes each).
 __host__ __device__ __forceinline__ SmemLayout smem_layout(int nlay, int ngas, int nband, int ncloud_vals, int NW,
                                                            int nmaps, int CL, int nbands_per_group, int nscal,
-                                                           int NWloc = -1)
+                                                           size_t rec_bytes, int NWloc = -1)
 {
     if (NWloc < 0) NWloc = NW;
     SmemLayout L;
@@ -351,7 +457,7 @@ __host__ __device__ __forceinline__ SmemLayout smem_layout(int nlay, int ngas, i
     L.maps = align16(L.cloud + sizeof(float) * size_t(ncloud_vals) * nband * nlay);
     L.sfc = align16(L.maps + sizeof(float4) * size_t(NW) * 32 * nmaps);
     L.recs = align16(L.sfc + sizeof(float) * 64);
-    L.total = align16(L.recs + sizeof(Rec) * size_t(NWloc) * CL * nbands_per_group);
+    L.total = align16(L.recs + rec_bytes * size_t(NWloc) * CL * nbands_per_group);
     return L;
 }
 

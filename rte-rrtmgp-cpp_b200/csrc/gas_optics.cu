@@ -133,15 +133,16 @@ gas_optics_sw_kernel(const KdistView<T> k, const GasSet<T> gases, int ncol, int 
     }
 }
 
-// FP32 variants on the corner-packed tables of the fused kernels (KdistView::kmaj4, pfrac4,
-// kmin2, krayl2, minor_g).  Same thread mapping and outputs; per (column, layer, g-point) the
-// major interpolation is two 16-byte loads instead of eight 4-byte ones (the Planck fraction
-// likewise), each minor interval one 8-byte pair per eta corner, and the sum over minor
-// intervals stays in registers instead of a shared-memory accumulator.  The per-band weights
-// are the records of the fused kernels (fused::record_weights) held in registers.  The minor
-// scalings are computed once per (column, layer) for every scaling kind (not per band) and
-// are indexed per g-point, so they sit in shared memory, one column of max_nscal values per
-// thread (stride kThreads: no bank conflicts).
+// FP32 variants on the corner-packed tables (KdistView::kmaj4, pfrac4, kmin2, krayl2, minor_g).  Same
+// thread mapping and outputs; per (column, layer, g-point) the major interpolation is two
+// 16-byte loads instead of eight 4-byte ones (the Planck fraction likewise), each minor
+// interval one 8-byte pair per eta corner, and the sum over minor intervals stays in registers
+// instead of a shared-memory accumulator.  The per-band weights (PackedWeights) stay in
+// registers.  The minor scalings are computed once per (column, layer) for every scaling kind
+// (not per band) and are indexed per g-point, so they sit in shared memory, one column of
+// max_nscal values per thread (stride kThreads: no bank conflicts).  All intervals of a g-point in
+// one 256-bit row, always loaded, were slower here: 628 -> 906 us (LW) and 398 -> 589 us (SW) at
+// 4096 x 91; the absent intervals' zeros take the load return path and registers too.
 // Usable when the tables satisfy the fused kernels' layout conditions (packed_tables_ok).
 // I32: every (column, layer, g-point) offset fits in 31 bits (packed_index32), so the output
 // offsets are 32-bit (one multiply-add per store address instead of 64-bit arithmetic and
@@ -151,9 +152,76 @@ __host__ __device__ inline size_t packed_smem_bytes(int ngas, int nscal)
     return sizeof(float) * size_t(ngas + 1 + nscal) * kThreads;
 }
 
+// Interpolation weights of one (layer, band) (interpolation_kernel,
+// gas_optics_rrtmgp_kernels.cu:256-291) with its table rows.
+struct PackedWeights {
+    int kx, ky;            // kmaj4 / pfrac4 rows of (t0, p0, e0), (t1, p0, e1)
+    int kz, kw;            // kmin2 rows of (t0, e0), (t1, e1)
+    int r0, r1;            // krayl2 rows of (a, t0, e0), (a, t1, e1)
+    float4 maj0, maj1;     // col_mix x fmajor (major absorption weights)
+    float4 pl0, pl1;       // fmajor (Planck fractions)
+    float4 fm;             // fminor (minor and Rayleigh weights)
+};
+
+__device__ __forceinline__ PackedWeights packed_weights(const KdistView<float>& k, const LayerInterp<float>& li,
+                                                        const float* cg, int cgs, int b)
+{
+    PackedWeights R;
+    const int a = li.itropo;
+    const FlavorWeights<float> fw = flavor_weights(k, k.band_flav[2 * b + a], li, cg, cgs);
+    const int ne1 = k.neta - 1, np = k.npres;
+    const int p0 = li.jp + a - 1;
+    R.kx = (((li.jt - 1) * np + p0) * ne1 + (fw.j0 - 1)) * k.ngpt;
+    R.ky = ((li.jt * np + p0) * ne1 + (fw.j1 - 1)) * k.ngpt;
+    const int nc = k.ncontrib[a] > 0 ? k.ncontrib[a] : 1;
+    // kmin2 rows; the Rayleigh rows (krayl2, [a][t][eta][g]) follow the same (t, eta) corners.
+    R.kz = ((li.jt - 1) * ne1 + (fw.j0 - 1)) * nc;
+    R.kw = (li.jt * ne1 + (fw.j1 - 1)) * nc;
+    R.r0 = ((a * k.ntemp + li.jt - 1) * ne1 + (fw.j0 - 1)) * k.ngpt;
+    R.r1 = ((a * k.ntemp + li.jt) * ne1 + (fw.j1 - 1)) * k.ngpt;
+    const float fp = li.fpress, f1 = 1.f - li.fpress;
+    R.pl0 = make_float4(f1 * fw.fm[0], f1 * fw.fm[1], fp * fw.fm[0], fp * fw.fm[1]);
+    R.pl1 = make_float4(f1 * fw.fm[2], f1 * fw.fm[3], fp * fw.fm[2], fp * fw.fm[3]);
+    R.maj0 = make_float4(fw.cm[0] * R.pl0.x, fw.cm[0] * R.pl0.y, fw.cm[0] * R.pl0.z, fw.cm[0] * R.pl0.w);
+    R.maj1 = make_float4(fw.cm[1] * R.pl1.x, fw.cm[1] * R.pl1.y, fw.cm[1] * R.pl1.z, fw.cm[1] * R.pl1.w);
+    R.fm = make_float4(fw.fm[0], fw.fm[1], fw.fm[2], fw.fm[3]);
+    return R;
+}
+
+// Code n of g-point g's minor-interval list (minor_g / minor_gx; n < count, or a code that
+// repeats the first one for n < 3).
+__device__ __forceinline__ int minor_code_at(const KdistView<float>& k, int a, const int4& mg, int g, int n)
+{
+    if (n < 3) return n == 0 ? mg.y : (n == 1 ? mg.z : mg.w);
+    return n < mg.x ? __ldg(k.minor_gx[a] + size_t(g) * k.minor_gx_stride + (n - 3)) : mg.y;
+}
+
+// Absorption optical depth of g-point g: major (corners c0, c1) plus the mg.x minor intervals
+// covering g (minor_g list), as gas_optical_depths_major/minor.  sc: the layer's scalings, kind sid
+// at sc[sid * sst].  DENSE: tables with more than three intervals over some g-point; the loop
+// over the further ones is compiled only then.
+template <bool DENSE>
+__device__ __forceinline__ float packed_tau(const KdistView<float>& k, const PackedWeights& R, int a, int g,
+                                            const int4& mg, const float4& c0, const float4& c1, const float* sc, int sst)
+{
+    float tau = fused::dot4(R.maj0, c0) + fused::dot4(R.maj1, c1);
+    const float2* kn = k.kmin2[a];
+    auto term = [&](int code) {
+        const int c = code >> kScalBits;
+        const float2 lo = __ldg(kn + (R.kz + c)), hi = __ldg(kn + (R.kw + c));
+        tau += sc[(code & (kMaxScal - 1)) * sst] * (R.fm.x * lo.x + R.fm.y * lo.y + R.fm.z * hi.x + R.fm.w * hi.y);
+    };
+#pragma unroll
+    for (int n = 0; n < 3; ++n)
+        if (n < mg.x) term(n == 0 ? mg.y : (n == 1 ? mg.z : mg.w));
+    if constexpr (DENSE)
+        for (int n = 3; n < mg.x; ++n) term(minor_code_at(k, a, mg, g, n));
+    return tau;
+}
+
 inline bool packed_tables_ok(const KdistView<float>& v, bool lw)
 {
-    return fused::fused_layout_ok(v, !lw, 1 << 30) && v.minor_g[0] && v.minor_g[1];
+    return fused::fused_layout_ok(v, !lw, 1 << 30);
 }
 
 inline bool packed_index32(int ncol, int nlay, int ngpt)
@@ -165,21 +233,6 @@ inline bool packed_index32(int ncol, int nlay, int ngpt)
 __device__ __forceinline__ int4 next_minor_row(const int4* mgt, int g, int ngpt)
 {
     return g < ngpt ? __ldg(mgt + g) : make_int4(0, 0, 0, 0);
-}
-
-__device__ __forceinline__ fused::LayerState thread_layer_state(const LayerInterp<float>& li, float p, float t)
-{
-    fused::LayerState s;
-    s.jt = li.jt;
-    s.jp = li.jp;
-    s.itropo = li.itropo;
-    s.pad = 0;
-    s.ftemp = li.ftemp;
-    s.fpress = li.fpress;
-    s.p = p;
-    s.t = t;
-    s.t_top = s.t_bot = s.dp = s.pad2 = 0.f;
-    return s;
 }
 
 template <bool DENSE, bool I32>
@@ -205,7 +258,7 @@ gas_optics_lw_packed_kernel(const KdistView<float> k, const GasSet<float> gases,
 
     const float p = play[cl], t = tlay[cl];
     fill_col_gas(k, gases, ncol, nlay, icol, ilay, plev, col_dry_in, cg, kThreads);
-    const fused::LayerState s = thread_layer_state(layer_interp(k, p, t), p, t);
+    const LayerInterp<float> s = layer_interp(k, p, t);
     for (int sid = 0; sid < k.nscal[s.itropo]; ++sid)
         scal[sid * kThreads] = fused::kind_scaling(k, s.itropo, sid, cg, kThreads, p, t);
 
@@ -222,9 +275,7 @@ gas_optics_lw_packed_kernel(const KdistView<float> k, const GasSet<float> gases,
     int4 nx = __ldg(mgt);
     for (int b = 0; b < k.nband; ++b) {
         const int g0 = k.band_lims[2 * b], g1 = k.band_lims[2 * b + 1];
-        fused::Rec R;
-        fused::record_weights(k, R, s, cg, kThreads, b);
-        const float4 wp0 = R.wpl0, wp1 = R.wpl1;
+        const PackedWeights R = packed_weights(k, s, cg, kThreads, b);
 
         const float* tp = k.totplnk + size_t(b) * k.nplanck;
         const float pl = interpolate1D(t, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp);
@@ -240,11 +291,10 @@ gas_optics_lw_packed_kernel(const KdistView<float> k, const GasSet<float> gases,
         for (int g = g0; g < g1; ++g) {
             const int4 mg = nx;
             nx = next_minor_row(mgt, g + 1, k.ngpt);
-            const float ta = fused::tau_abs<DENSE>(k, R, g, mg, mg.x, scal, kThreads);
-            const float4 p0 = __ldg(k.pfrac4 + (R.kb.x + g));
-            const float4 p1 = __ldg(k.pfrac4 + (R.kb.y + g));
-            const float pfrac = (wp0.x * p0.x + wp0.y * p0.y + wp0.z * p0.z + wp0.w * p0.w) +
-                                (wp1.x * p1.x + wp1.y * p1.y + wp1.z * p1.z + wp1.w * p1.w);
+            const float ta = packed_tau<DENSE>(k, R, s.itropo, g, mg, __ldg(k.kmaj4 + (R.kx + g)),
+                                               __ldg(k.kmaj4 + (R.ky + g)), scal, kThreads);
+            const float4 p0 = __ldg(k.pfrac4 + (R.kx + g)), p1 = __ldg(k.pfrac4 + (R.ky + g));
+            const float pfrac = fused::dot4(R.pl0, p0) + fused::dot4(R.pl1, p1);
             const Idx o = cl + Idx(g) * ncl;
             tau[o] = ta;
             lay_src[o] = pfrac * pl;
@@ -279,7 +329,7 @@ gas_optics_sw_packed_kernel(const KdistView<float> k, const GasSet<float> gases,
 
     const float p = play[cl], t = tlay[cl];
     fill_col_gas(k, gases, ncol, nlay, icol, ilay, plev, col_dry_in, cg, kThreads);
-    const fused::LayerState s = thread_layer_state(layer_interp(k, p, t), p, t);
+    const LayerInterp<float> s = layer_interp(k, p, t);
     for (int sid = 0; sid < k.nscal[s.itropo]; ++sid)
         scal[sid * kThreads] = fused::kind_scaling(k, s.itropo, sid, cg, kThreads, p, t);
     const float col_rayl = cg[k.idx_h2o * kThreads] + cg[0];
@@ -289,17 +339,16 @@ gas_optics_sw_packed_kernel(const KdistView<float> k, const GasSet<float> gases,
     int4 nx = __ldg(mgt);
     for (int b = 0; b < k.nband; ++b) {
         const int g0 = k.band_lims[2 * b], g1 = k.band_lims[2 * b + 1];
-        fused::Rec R;
-        fused::record_weights(k, R, s, cg, kThreads, b);
-        const int kr0 = R.kr[0], kr1 = R.kr[1];
+        const PackedWeights R = packed_weights(k, s, cg, kThreads, b);
         // two g-points per iteration, as the longwave kernel
 #pragma unroll 2
         for (int g = g0; g < g1; ++g) {
             const int4 mg = nx;
             nx = next_minor_row(mgt, g + 1, k.ngpt);
-            const float ta = fused::tau_abs<DENSE>(k, R, g, mg, mg.x, scal, kThreads);
-            const float2 r0 = __ldg(k.krayl2 + (kr0 + g));
-            const float2 r1 = __ldg(k.krayl2 + (kr1 + g));
+            const float ta = packed_tau<DENSE>(k, R, s.itropo, g, mg, __ldg(k.kmaj4 + (R.kx + g)),
+                                               __ldg(k.kmaj4 + (R.ky + g)), scal, kThreads);
+            const float2 r0 = __ldg(k.krayl2 + (R.r0 + g));
+            const float2 r1 = __ldg(k.krayl2 + (R.r1 + g));
             const float tr = (R.fm.x * r0.x + R.fm.y * r0.y + R.fm.z * r1.x + R.fm.w * r1.y) * col_rayl;
             const float tt = ta + tr;
             const Idx o = cl + Idx(g) * ncl;

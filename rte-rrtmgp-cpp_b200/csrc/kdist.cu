@@ -238,11 +238,14 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
     v.max_group_bands = max_gb;
     a.add(gb0, &v.group_band0);
 
-    // Corner-packed tables for the fused FP32 kernels.
+    // Corner-packed tables of the FP32 kernels (see KdistView).
     v.max_minor_per_g = 0;
     v.minor_gx_stride = 0;
-    std::vector<float4> km4, pf4;
+    v.nminor_units = 1;
+    std::vector<float4> km4, pf4, kn4;
+    std::vector<Tab8> kp8;
     std::vector<float2> kn2[2], kr2;
+    std::vector<int2> ms;
     std::vector<int4> mg[2];
     std::vector<int> mgx[2];
     if (std::is_same<T, float>::value) {
@@ -259,7 +262,11 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
                                             at(it, ip + 1, ie + 1, ig));
         };
         pack4(t->kmajor, km4);
-        if (t->planck_frac) pack4(t->planck_frac, pf4);
+        if (t->planck_frac) {
+            pack4(t->planck_frac, pf4);
+            kp8.resize(km4.size());
+            for (size_t i = 0; i < km4.size(); ++i) kp8[i] = {km4[i], pf4[i]};
+        }
         for (int atm = 0; atm < 2; ++atm) {
             const MinorHost& m = mh[atm];
             const int nc = std::max(m.ncontrib, 1);
@@ -310,9 +317,44 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
                                             float(r[(size_t(it) * ne + ie + 1) * ng + ig]));
             }
         }
+        // Minor intervals of the fused kernels (KdistView::kmin4, minor_s).
+        const int r0 = info.is_longwave ? 0 : 1;   // the shortwave's first pair is the Rayleigh coefficient's
+        const int nu = std::max(1, (v.max_minor_per_g + r0 + 1) / 2);
+        v.nminor_units = nu;
+        ms.assign(size_t(2) * nu * ng, make_int2(0, 0));
+        kn4.assign(size_t(2) * nt * (ne - 1) * nu * ng, make_float4(0.f, 0.f, 0.f, 0.f));
+        for (int atm = 0; atm < 2; ++atm) {
+            const MinorHost& m = mh[atm];
+            const int nc = std::max(m.ncontrib, 1);
+            const double* rayl = !info.has_rayleigh ? nullptr : (atm == 0 ? t->rayl_lower : t->rayl_upper);
+            for (int u = 0; u < nu; ++u)
+                for (int g = 0; g < ng; ++g) {
+                    const std::vector<int>& c = codes[atm][g];
+                    int sids = 0;
+                    for (int q = 0; q < 2; ++q) {
+                        const int n = 2 * u + q - r0;   // interval of this pair, -1: Rayleigh
+                        if (n >= 0 && n < int(c.size())) sids |= (c[n] & (kMaxScal - 1)) << (8 * q);
+                        if (n >= int(c.size()) || (n < 0 && !rayl)) continue;
+                        for (int it = 0; it < nt; ++it)
+                            for (int ie = 0; ie < ne - 1; ++ie) {
+                                float4& o = kn4[(((size_t(atm) * nt + it) * (ne - 1) + ie) * nu + u) * ng + g];
+                                for (int e = 0; e < 2; ++e) {
+                                    const size_t row = size_t(it) * ne + ie + e;
+                                    const float v1 = n < 0 ? float(rayl[row * ng + g])
+                                                           : float(m.kminor[row * nc + (c[n] >> kScalBits)]);
+                                    (q == 0 ? (e == 0 ? o.x : o.y) : (e == 0 ? o.z : o.w)) = v1;
+                                }
+                            }
+                    }
+                    ms[(size_t(atm) * nu + u) * ng + g] = make_int2(sids, int(c.size()));
+                }
+        }
     }
+    a.add(kn4, &v.kmin4);
+    a.add(ms, &v.minor_s);
     a.add(km4, &v.kmaj4);
     a.add(pf4, &v.pfrac4);
+    a.add(kp8, &v.kmp8);
     a.add(kn2[0], &v.kmin2[0]);
     a.add(kn2[1], &v.kmin2[1]);
     a.add(kr2, &v.krayl2);

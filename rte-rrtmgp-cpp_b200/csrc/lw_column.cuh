@@ -54,16 +54,16 @@ struct LwGridIo {
     __device__ __forceinline__ const CloudArgs& cloud() const { return cld_; }
 };
 
-__device__ __forceinline__ void build_lw_record(const KdistView<float>& k, Rec& R, const LayerState& s,
+__device__ __forceinline__ void build_lw_record(const KdistView<float>& k, LwRec& R, const LayerState& s,
                                                 const float* cg, int nlay, int b, float tau_cld, bool bottom,
                                                 float tsfc)
 {
-    record_weights(k, R, s, cg, nlay, b);
     const float* tp = k.totplnk + size_t(b) * k.nplanck;
+    record_weights(k, R, s, cg, nlay, b,
+                   bottom ? interpolate1D(tsfc, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp) : 0.f);
     R.aux = make_float4(interpolate1D(s.t, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp),
                         interpolate1D(s.t_top, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp),
                         interpolate1D(s.t_bot, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp), tau_cld);
-    R.aux2 = bottom ? interpolate1D(tsfc, k.temp_ref_min, k.totplnk_delta, k.nplanck, tp) : 0.f;
 }
 
 // One column by the warps that context cx names (cx.nwarps() warps of CL layers each,
@@ -87,7 +87,7 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
     // sized by capacity (NWloc CL layers), the same in every CTA of a cluster: the chunk maps
     // stored into another CTA's shared memory land at the offset this CTA uses
     const SmemLayout SL = smem_layout(NWloc * CL, k.ngas, nband, 1, cx.nwarps(), 2, CL,
-                                      k.max_group_bands * (P2 ? 2 : 1), k.max_nscal, NWloc);
+                                      k.max_group_bands * (P2 ? 2 : 1), k.max_nscal, sizeof(LwRec), NWloc);
     unsigned char* const smem_raw = cx.smem();
     LayerState* st = reinterpret_cast<LayerState*>(smem_raw + SL.state);
     float* sm_cg = reinterpret_cast<float*>(smem_raw + SL.cg);
@@ -97,7 +97,7 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
     // start the next group while others still read this group's (one barrier per group)
     float4* const sm_maps0 = reinterpret_cast<float4*>(smem_raw + SL.maps);
     float* const sm_sfc0 = reinterpret_cast<float*>(smem_raw + SL.sfc);
-    Rec* const recs0 = reinterpret_cast<Rec*>(smem_raw + SL.recs) + cx.lwarp() * CL * k.max_group_bands;
+    LwRec* const recs0 = reinterpret_cast<LwRec*>(smem_raw + SL.recs) + cx.lwarp() * CL * k.max_group_bands;
     const int rbuf = NWloc * CL * k.max_group_bands;   // records per buffer
 
     bool top_at_1;
@@ -126,6 +126,9 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
     layer_minor_scalings(k, st, sm_cg, NL, sm_sc, NL, cx.tid(), cx.nthreads());
     cx.sync();
 
+    // bit i: layer i of this warp's chunk is in the upper atmosphere
+    const unsigned upper = __ballot_sync(0xffffffffu, lane < CL && cx.warp() * CL + lane < io.nlay() &&
+                                                          st[cx.warp() * CL - L0 + (lane < CL ? lane : 0)].itropo);
     const float D = 1.66f;                 // single-angle secant (Rte_lw.cpp:101-113)
     const int ngpt = k.ngpt;
     double acc_lev = 0.0, acc_div = 0.0, acc_bot_up = 0.0, acc_bot_dn = 0.0;
@@ -139,13 +142,10 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
         const int b0 = k.group_band0[gg];
         const int gband = gv ? k.gpt2band[g] : b0;
         const int slot = gband - b0;
-        const int4 mg0 = minor_entry(k.minor_g[0], g, gv);
-        const int4 mg1 = minor_entry(k.minor_g[1], g, gv);
-        const int nm0 = __reduce_max_sync(0xffffffffu, mg0.x);
-        const int nm1 = __reduce_max_sync(0xffffffffu, mg1.x);
+        const MinorRef mr0 = minor_ref(k, 0, g, gv), mr1 = minor_ref(k, 1, g, gv);
 
         // 1. records of this warp's chunk
-        Rec* const recs = recs0 + (P2 ? (gg & 1) : 0) * rbuf;
+        LwRec* const recs = recs0 + (P2 ? (gg & 1) : 0) * rbuf;
         if (!P2 || (gg & 1) == 0) {
             const int nrec = CL * k.max_group_bands;
             for (int t = lane; t < (P2 ? 2 : 1) * nrec; t += 32) {
@@ -169,16 +169,16 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
             const int j = j0 + i;
             omt[i] = 0.f; sdn[i] = 0.f; sup[i] = 0.f;
             if (j < nlay && gv) {
-                const Rec& R = recs[slot * CL + i];
-                const float tau =
-                    tau_abs<DENSE>(k, R, g, R.a ? mg1 : mg0, R.a ? nm1 : nm0, sm_sc + (j - L0) * k.max_nscal) +
-                    R.aux.w;
-                const float4 p0 = __ldg(k.pfrac4 + (R.kb.x + g));
-                const float4 p1 = __ldg(k.pfrac4 + (R.kb.y + g));
-                const float pfrac = (R.wpl0.x * p0.x + R.wpl0.y * p0.y + R.wpl0.z * p0.z + R.wpl0.w * p0.w) +
-                                    (R.wpl1.x * p1.x + R.wpl1.y * p1.y + R.wpl1.z * p1.z + R.wpl1.w * p1.w);
+                const LwRec& R = recs[slot * CL + i];
+                GasRows r;
+                const int a = (upper >> i) & 1;
+                const MinorRef mr = a ? mr1 : mr0;
+                load_rows<false>(gas_tab(k), R.kb, g, mr.nmax, r);
+                const float tau = tau_abs<false, DENSE>(gas_tab(k), R, a, g, r, mr, sm_sc + (j - L0) * k.max_nscal) +
+                                  R.aux.w;
+                const float pfrac = planck_fraction(R, r);
                 lw_layer_fast(tau, D, pfrac * R.aux.x, pfrac * R.aux.z, pfrac * R.aux.y, omt[i], sdn[i], sup[i]);
-                if (j == nlay - 1) cx.put(&sm_sfc[lane], pfrac * R.aux2);
+                if (j == nlay - 1) cx.put(&sm_sfc[lane], pfrac * R.mix.w);
             } else if (j == nlay - 1) {
                 cx.put(&sm_sfc[lane], 0.f);
             }

@@ -77,7 +77,7 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
     const int NWloc = cx.nthreads() >> 5;
     // sized by capacity (NWloc CL layers), the same in every CTA of a cluster (as lw_forward_column)
     const SmemLayout SL = smem_layout(NWloc * CL, k.ngas, nband, with_aer ? 4 : 0, cx.nwarps(), 3, CL,
-                                      k.max_group_bands * (P2 ? 2 : 1), k.max_nscal, NWloc);
+                                      k.max_group_bands * (P2 ? 2 : 1), k.max_nscal, sizeof(SwRec), NWloc);
     unsigned char* const smem_raw = cx.smem();
     LayerState* st = reinterpret_cast<LayerState*>(smem_raw + SL.state);
     float* sm_cg = reinterpret_cast<float*>(smem_raw + SL.cg);
@@ -85,7 +85,7 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
     float* sm_pt = reinterpret_cast<float*>(smem_raw + SL.maps);                            // [NW][32]
     float4* sm_comp = reinterpret_cast<float4*>(smem_raw + SL.maps) + cx.nwarps() * 32;     // [NW][32]
     float* sm_compd = reinterpret_cast<float*>(sm_comp + cx.nwarps() * 32);                 // [NW][32]
-    Rec* const recs0 = reinterpret_cast<Rec*>(smem_raw + SL.recs) + cx.lwarp() * CL * k.max_group_bands;
+    SwRec* const recs0 = reinterpret_cast<SwRec*>(smem_raw + SL.recs) + cx.lwarp() * CL * k.max_group_bands;
     const int rbuf = NWloc * CL * k.max_group_bands;   // records per buffer
 
     bool top_at_1;
@@ -112,6 +112,9 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
     }
     cx.sync();
 
+    // bit i: layer i of this warp's chunk is in the upper atmosphere
+    const unsigned upper = __ballot_sync(0xffffffffu, lane < CL && cx.warp() * CL + lane < io.nlay() &&
+                                                          st[cx.warp() * CL - L0 + (lane < CL ? lane : 0)].itropo);
     const int ngpt = k.ngpt;
     constexpr int SH = (CL == 16) ? 0 : 1;          // lane L holds reduced value L >> SH
     double acc_a = 0.0, acc_b = 0.0, acc_c = 0.0;   // see the output section
@@ -124,12 +127,9 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
         const int b0 = k.group_band0[gg];
         const int gband = gv ? k.gpt2band[g] : b0;
         const int slot = gband - b0;
-        const int4 mg0 = minor_entry(k.minor_g[0], g, gv);
-        const int4 mg1 = minor_entry(k.minor_g[1], g, gv);
-        const int nm0 = __reduce_max_sync(0xffffffffu, mg0.x);
-        const int nm1 = __reduce_max_sync(0xffffffffu, mg1.x);
+        const MinorRef mr0 = minor_ref(k, 0, g, gv), mr1 = minor_ref(k, 1, g, gv);
 
-        Rec* const recs = recs0 + (P2 ? (gg & 1) : 0) * rbuf;
+        SwRec* const recs = recs0 + (P2 ? (gg & 1) : 0) * rbuf;
         if (!P2 || (gg & 1) == 0) {
             const int nrec = CL * k.max_group_bands;
             for (int t = lane; t < (P2 ? 2 : 1) * nrec; t += 32) {
@@ -157,12 +157,13 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
             const int j = j0 + i;
             float R = 0.f, T = 1.f, Rdir = 0.f, Tdir = 0.f, Tn = 1.f, adif = 0.f, adir = 0.f;
             if (j < nlay && gv) {
-                const Rec& Rc = recs[slot * CL + i];
-                const float ta =
-                    tau_abs<DENSE>(k, Rc, g, Rc.a ? mg1 : mg0, Rc.a ? nm1 : nm0, sm_sc + (j - L0) * k.max_nscal);
-                const float2 r0 = __ldg(k.krayl2 + (Rc.kr[0] + g));
-                const float2 r1 = __ldg(k.krayl2 + (Rc.kr[1] + g));
-                const float tr = (Rc.fm.x * r0.x + Rc.fm.y * r0.y + Rc.fm.z * r1.x + Rc.fm.w * r1.y) * Rc.aux.x;
+                const SwRec& Rc = recs[slot * CL + i];
+                GasRows r;
+                const int a = (upper >> i) & 1;
+                const MinorRef mr = a ? mr1 : mr0;
+                load_rows<true>(gas_tab(k), Rc.kb, g, mr.nmax, r);
+                const float ta = tau_abs<true, DENSE>(gas_tab(k), Rc, a, g, r, mr, sm_sc + (j - L0) * k.max_nscal);
+                const float tr = dot4(Rc.fm, rayleigh_corners(r)) * Rc.aux.x;
                 const float tau = ta + tr + Rc.aux.y;
                 const float ts = tr + Rc.aux.z;
                 float w0 = 0.f, omw = 1.f;

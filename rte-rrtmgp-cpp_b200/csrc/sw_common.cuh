@@ -145,7 +145,7 @@ __device__ __forceinline__ void sw_layer_fast(float tau, float w0, float omw, fl
 }
 
 // aer: the (layer, band) aerosol values of aerosol_point, or NULL without aerosols.
-__device__ __forceinline__ void build_sw_record(const KdistView<float>& k, Rec& R, const LayerState& s,
+__device__ __forceinline__ void build_sw_record(const KdistView<float>& k, SwRec& R, const LayerState& s,
                                                 const float* cg, int nlay, int b, const SwCloudArgs& cld,
                                                 size_t cl, const float4* aer = nullptr)
 {
