@@ -82,9 +82,13 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
     LayerState* st = reinterpret_cast<LayerState*>(smem_raw + SL.state);
     float* sm_cg = reinterpret_cast<float*>(smem_raw + SL.cg);
     float* sm_sc = reinterpret_cast<float*>(smem_raw + SL.scal);   // [layer][scaling kind]
-    float* sm_pt = reinterpret_cast<float*>(smem_raw + SL.maps);                            // [NW][32]
-    float4* sm_comp = reinterpret_cast<float4*>(smem_raw + SL.maps) + cx.nwarps() * 32;     // [NW][32]
-    float* sm_compd = reinterpret_cast<float*>(sm_comp + cx.nwarps() * 32);                 // [NW][32]
+    // chunk exchange, [NW][32] each, in 48 bytes per (chunk, lane): direct transmission (4),
+    // sm_below (8), composite (16 + 4), sm_above (8)
+    float* sm_pt = reinterpret_cast<float*>(smem_raw + SL.maps);
+    float2* sm_below = reinterpret_cast<float2*>(sm_pt + cx.nwarps() * 32);
+    float4* sm_comp = reinterpret_cast<float4*>(smem_raw + SL.maps) + cx.nwarps() * 32;
+    float* sm_compd = reinterpret_cast<float*>(sm_comp + cx.nwarps() * 32);
+    float2* sm_above = reinterpret_cast<float2*>(sm_compd + cx.nwarps() * 32);
     SwRec* const recs0 = reinterpret_cast<SwRec*>(smem_raw + SL.recs) + cx.lwarp() * CL * k.max_group_bands;
     const int rbuf = NWloc * CL * k.max_group_bands;   // records per buffer
 
@@ -203,8 +207,9 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
         const float toa = gv ? __ldg(k.solar_source + g) * tsi * mu0 : 0.f;
         float dtop = toa;
         for (int c = 0; c < w; ++c) dtop *= sm_pt[c * 32 + lane];
-        float dsfc = dtop;
-        for (int c = w; c < NW; ++c) dsfc *= sm_pt[c * 32 + lane];
+        float dsfc = dtop;   // direct flux at the surface, where it is used
+        if (w == 0 || w == NW - 1)
+            for (int c = w; c < NW; ++c) dsfc *= sm_pt[c * 32 + lane];
         {
             float v[2 * CL];
 #pragma unroll
@@ -219,39 +224,59 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
         cx.put(&sm_compd[w * 32 + lane], cD * dtop);
         cx.sync();
 
-        // 3. albedo and source at this chunk's bottom; incident diffuse flux at its top.  Chunk 0's
-        //    warp scans the composites of all chunks: from the surface up, the albedo and source
-        //    at each chunk bottom and the chunk's transfer of the diffuse flux (flux at its bottom
-        //    = F * flux at its top + G); then from the top down, the diffuse flux entering each
-        //    chunk (no diffuse flux at the top of the atmosphere).  The results replace the
-        //    composites (each slot read before it is rewritten, through put for every CTA of a
-        //    cluster), and every warp reads its own chunk's after one more barrier: with every
-        //    warp scanning the chunks itself the scans were O(chunks^2) per group.
+        // 3. albedo and source at this chunk's bottom; incident diffuse flux at its top.  Two warps scan the
+        //    chunk composites while the others wait: chunk 0's from the surface up, the albedo and
+        //    upward source of everything below each chunk's bottom (sm_below); chunk 1's from the
+        //    top down, the reflectance from below and the downward source of everything above it
+        //    (sm_above: no diffuse flux at the top of the atmosphere).  At an interface the two
+        //    sides close: f_dn = (D + Rd src) / (1 - Rd alb).  Both scans are chains of NW
+        //    divisions on which the whole CTA waits, so they run side by side and load a chunk ahead
+        //    (one warp doing the upward scan and then walking the fluxes back down: 8192 x 128
+        //    SW forward 4.05 -> 3.86 ms, with the layer transfers below kept from pass 2); with every warp scanning all chunks itself they were
+        //    O(chunks^2) instructions per group.
         const float ad = gv ? __ldg(io.alb_dir() + gband + size_t(cx.icol()) * nband) : 0.f;
         const float af = gv ? __ldg(io.alb_dif() + gband + size_t(cx.icol()) * nband) : 0.f;
         if (w == 0) {
             float alb = af, src = dsfc * ad;
+            float4 m = sm_comp[(NW - 1) * 32 + lane];
+            float D = sm_compd[(NW - 1) * 32 + lane];
             for (int c = NW - 1; c >= 0; --c) {
-                const float4 m = sm_comp[c * 32 + lane];
-                const float D = sm_compd[c * 32 + lane];
-                const float den = fast_div(1.f, fmaf(-m.y, alb, 1.f));
-                cx.put(&sm_comp[c * 32 + lane], make_float4(alb, src, m.z * den, fmaf(m.y, src, D) * den));
-                const float nalb = m.x + m.z * m.z * alb * den;
-                src = m.w + m.z * fmaf(alb, D, src) * den;
-                alb = nalb;
+                cx.put(&sm_below[c * 32 + lane], make_float2(alb, src));
+                const int cn = max(c - 1, 0) * 32 + lane;
+                const float4 mn = sm_comp[cn];
+                const float Dn = sm_compd[cn];
+                const float t = m.z * fast_div(1.f, fmaf(-m.y, alb, 1.f));
+                src = fmaf(t, fmaf(alb, D, src), m.w);
+                alb = fmaf(t * m.z, alb, m.x);
+                m = mn;
+                D = Dn;
             }
-            float f = 0.f;
-            for (int c = 0; c < NW; ++c) {
-                cx.put(&sm_compd[c * 32 + lane], f);
-                const float4 r = sm_comp[c * 32 + lane];
-                f = fmaf(r.z, f, r.w);
+        } else if (w == 1) {
+            float Rd = 0.f, D = 0.f;
+            float4 m = sm_comp[lane];
+            float Dc = sm_compd[lane];
+            for (int c = 0; c < NW - 1; ++c) {
+                const int cn = (c + 1) * 32 + lane;
+                const float4 mn = sm_comp[cn];
+                const float Dn = sm_compd[cn];
+                const float t = m.z * fast_div(1.f, fmaf(-Rd, m.x, 1.f));
+                D = fmaf(t, fmaf(Rd, m.w, D), Dc);
+                Rd = fmaf(t * m.z, Rd, m.y);
+                cx.put(&sm_above[c * 32 + lane], make_float2(Rd, D));
+                m = mn;
+                Dc = Dn;
             }
         }
         cx.sync();
-        const float4 own = sm_comp[w * 32 + lane];
-        const float alb_in = own.x, src_in = own.y, fb = sm_compd[w * 32 + lane];
+        const float alb_in = sm_below[w * 32 + lane].x, src_in = sm_below[w * 32 + lane].y;
+        float fb = 0.f;
+        if (w > 0) {
+            const float2 lo = sm_below[(w - 1) * 32 + lane], up = sm_above[(w - 1) * 32 + lane];
+            fb = fast_div(fmaf(up.x, lo.y, up.y), fmaf(-up.x, lo.x, 1.f));
+        }
 
-        // 4. pass 2 (bottom-up): albedo and upward source per level
+        // 4. pass 2 (bottom-up): albedo and upward source per level, and each layer's transfer of the
+        //    diffuse downward flux, f_dn(bottom) = vT f_dn(top) + vSd
         float vA[CL];
         {
             float a = alb_in, s = src_in;
@@ -259,9 +284,11 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
             for (int i = CL - 1; i >= 0; --i) {
                 const float su = vSu[i] * dtop, sd = vSd[i] * dtop;
                 const float den = fast_div(1.f, fmaf(-vR[i], a, 1.f));
-                const float na = vR[i] + vT[i] * vT[i] * a * den;
-                const float ns = su + vT[i] * fmaf(a, sd, s) * den;
-                vSd[i] = sd;
+                const float t = vT[i] * den;
+                const float na = vR[i] + t * vT[i] * a;
+                const float ns = su + t * fmaf(a, sd, s);
+                vT[i] = t;
+                vSd[i] = fmaf(vR[i], s, sd) * den;
                 vSu[i] = ns;
                 vA[i] = na;
                 a = na;
@@ -269,29 +296,27 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
             }
         }
         // pass 3 (top-down): diffuse fluxes and diffuse absorption
-        float vUp[2 * CL], vDn[2 * CL];
-        float fd = fb;
+        float vUp[2 * CL], vDn[CL];
+        float fd = fb, fu = fmaf(fb, vA[0], vSu[0]);
 #pragma unroll
         for (int i = 0; i < CL; ++i) {
             const float a_n = (i + 1 < CL) ? vA[i + 1] : alb_in;
             const float s_n = (i + 1 < CL) ? vSu[i + 1] : src_in;
-            const float fu = fmaf(fd, vA[i], vSu[i]);
-            const float den = fast_div(1.f, fmaf(-vR[i], a_n, 1.f));
-            const float fdn = (vT[i] * fd + vR[i] * s_n + vSd[i]) * den;
+            const float fdn = fmaf(vT[i], fd, vSd[i]);
             const float fun = fmaf(fdn, a_n, s_n);
             vUp[i] = fu;
             vUp[CL + i] = (fd + fun) * vAd[i];
             vDn[i] = fd;
-            vDn[CL + i] = 0.f;
             fd = fdn;
+            fu = fun;
         }
         if (w == NW - 1) {
             acc_sfc_dir += double(warp_sum(dsfc));
             acc_sfc_dn += double(warp_sum(fd));
-            acc_sfc_up += double(warp_sum(fmaf(fd, alb_in, src_in)));
+            acc_sfc_up += double(warp_sum(fu));
         }
         ReduceScatter<2 * CL, 16>::run(vUp, lane);
-        ReduceScatter<2 * CL, 16>::run(vDn, lane);
+        ReduceScatter<CL, 16>::run(vDn, lane);
         acc_b += double(vUp[0]);
         acc_c += double(vDn[0]);
     }
@@ -306,6 +331,7 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
     float* const flux_net = io.net();
     float* const heating_rate = io.hr();
     const int v = lane >> SH;
+    acc_c = __shfl_sync(0xffffffffu, acc_c, (2 * v << SH) & 31);   // reduced over CL values: lane L holds value L >> (SH + 1)
     if ((lane & ((1 << SH) - 1)) == 0) {
         if (v < CL) {
             const int jl = w * CL + v;
