@@ -186,6 +186,7 @@ struct rrtmgp_b200_kdist_t {
     double* d_solar64 = nullptr;
     int* d_flags = nullptr;   // range-check result word
     int device = 0;
+    int nsm = 0;              // multiprocessors of that device
 };
 
 struct rrtmgp_b200_cloud_t {

@@ -52,31 +52,75 @@ int find1(const std::vector<std::string>& v, const std::string& s)
     return -1;
 }
 
-// Packs host arrays into one device allocation (256-byte aligned sub-buffers).
+// Collects host arrays (which stay alive until upload) and device-only ones into one device
+// allocation (256-byte aligned sub-buffers).  Every array is copied from where it lies; gathering
+// them in one host buffer first and packing the corner tables on the host took half of the
+// handle's creation.
 struct Arena {
-    std::vector<char> host;
-    std::vector<std::pair<size_t, void**>> fixups;
+    struct Piece {
+        const void* src;   // NULL: device-only, or an empty array (zeroed)
+        size_t off, bytes;
+        void** dst;
+    };
+    std::vector<Piece> pieces;
+    size_t total = 0;
 
+    void place(const void* src, size_t bytes, void** dst)
+    {
+        const size_t off = (total + 255) & ~size_t(255);
+        pieces.push_back({src, off, bytes, dst});
+        total = off + bytes;
+    }
     template <typename U>
     void add(const std::vector<U>& v, const U** dst)
     {
-        size_t off = (host.size() + 255) & ~size_t(255);
-        host.resize(off + std::max<size_t>(v.size(), 1) * sizeof(U), 0);
-        if (!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * sizeof(U));
-        fixups.push_back({off, reinterpret_cast<void**>(const_cast<U**>(dst))});
+        place(v.empty() ? nullptr : v.data(), std::max<size_t>(v.size(), 1) * sizeof(U),
+              reinterpret_cast<void**>(const_cast<U**>(dst)));
+    }
+    // n elements (at least one) that a kernel fills after upload
+    template <typename U>
+    void reserve(size_t n, const U** dst)
+    {
+        place(nullptr, std::max<size_t>(n, 1) * sizeof(U), reinterpret_cast<void**>(const_cast<U**>(dst)));
     }
 
     int upload(std::vector<void*>& allocs)
     {
         void* d = nullptr;
-        if (cudaMalloc(&d, std::max<size_t>(host.size(), 256)) != cudaSuccess)
+        if (cudaMalloc(&d, std::max<size_t>(total, 256)) != cudaSuccess)
             return fail(RRTMGP_B200_ERR_ALLOC, "cudaMalloc of k-distribution tables failed");
-        RB_CUDA(cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice), "table upload");
         allocs.push_back(d);
-        for (auto& f : fixups) *f.second = static_cast<char*>(d) + f.first;
+        for (const Piece& p : pieces) {
+            void* const to = static_cast<char*>(d) + p.off;
+            if (p.src) RB_CUDA(cudaMemcpy(to, p.src, p.bytes, cudaMemcpyHostToDevice), "table upload");
+            else RB_CUDA(cudaMemset(to, 0, p.bytes), "table upload");
+            *p.dst = to;
+        }
         return RRTMGP_B200_OK;
     }
 };
+
+// kmaj4 / pfrac4 / kmp8 (KdistView) from the [t][p][eta][g] tables; pf, pf4 and both may be NULL.
+__global__ void pack_corners_kernel(int nt, int np, int ne, int ng, const float* __restrict__ km,
+                                    const float* __restrict__ pf, float4* __restrict__ km4, float4* __restrict__ pf4,
+                                    Tab8* __restrict__ both)
+{
+    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= size_t(nt) * np * (ne - 1) * ng) return;
+    const int g = int(i % ng);
+    size_t r = i / ng;
+    const int e = int(r % (ne - 1));
+    r /= ne - 1;
+    const int p = int(r % np), t = int(r / np);
+    const size_t o = ((size_t(t) * (np + 1) + p) * ne + e) * ng + g, dp = size_t(ne) * ng;
+    const float4 a = make_float4(km[o], km[o + ng], km[o + dp], km[o + dp + ng]);
+    km4[i] = a;
+    if (pf) {
+        const float4 b = make_float4(pf[o], pf[o + ng], pf[o + dp], pf[o + dp + ng]);
+        pf4[i] = b;
+        both[i] = Tab8{a, b};
+    }
+}
 
 template <typename T>
 std::vector<T> conv(const double* p, size_t n)
@@ -242,31 +286,13 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
     v.max_minor_per_g = 0;
     v.minor_gx_stride = 0;
     v.nminor_units = 1;
-    std::vector<float4> km4, pf4, kn4;
-    std::vector<Tab8> kp8;
+    std::vector<float4> kn4;
     std::vector<float2> kn2[2], kr2;
     std::vector<int2> ms;
     std::vector<int4> mg[2];
     std::vector<int> mgx[2];
     if (std::is_same<T, float>::value) {
-        const int nt = t->ntemp, np = t->npres, np1 = t->npres + 1, ne = t->neta, ng = t->ngpt;
-        auto pack4 = [&](const double* src, std::vector<float4>& dst) {
-            dst.resize(size_t(nt) * np * (ne - 1) * ng);
-            auto at = [&](int it, int ip, int ie, int ig) { return float(src[((size_t(it) * np1 + ip) * ne + ie) * ng + ig]); };
-            for (int it = 0; it < nt; ++it)
-                for (int ip = 0; ip < np; ++ip)
-                    for (int ie = 0; ie < ne - 1; ++ie)
-                        for (int ig = 0; ig < ng; ++ig)
-                            dst[((size_t(it) * np + ip) * (ne - 1) + ie) * ng + ig] =
-                                make_float4(at(it, ip, ie, ig), at(it, ip, ie + 1, ig), at(it, ip + 1, ie, ig),
-                                            at(it, ip + 1, ie + 1, ig));
-        };
-        pack4(t->kmajor, km4);
-        if (t->planck_frac) {
-            pack4(t->planck_frac, pf4);
-            kp8.resize(km4.size());
-            for (size_t i = 0; i < km4.size(); ++i) kp8[i] = {km4[i], pf4[i]};
-        }
+        const int nt = t->ntemp, ne = t->neta, ng = t->ngpt;
         for (int atm = 0; atm < 2; ++atm) {
             const MinorHost& m = mh[atm];
             const int nc = std::max(m.ncontrib, 1);
@@ -352,9 +378,11 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
     }
     a.add(kn4, &v.kmin4);
     a.add(ms, &v.minor_s);
-    a.add(km4, &v.kmaj4);
-    a.add(pf4, &v.pfrac4);
-    a.add(kp8, &v.kmp8);
+    const size_t nrow =
+        std::is_same<T, float>::value ? size_t(t->ntemp) * t->npres * (t->neta - 1) * t->ngpt : 0;
+    a.reserve(nrow, &v.kmaj4);
+    a.reserve(t->planck_frac ? nrow : 0, &v.pfrac4);
+    a.reserve(t->planck_frac ? nrow : 0, &v.kmp8);
     a.add(kn2[0], &v.kmin2[0]);
     a.add(kn2[1], &v.kmin2[1]);
     a.add(kr2, &v.krayl2);
@@ -362,7 +390,16 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
     a.add(mg[1], &v.minor_g[1]);
     a.add(mgx[0], &v.minor_gx[0]);
     a.add(mgx[1], &v.minor_gx[1]);
-    return a.upload(k->allocations);
+    const int st = a.upload(k->allocations);
+    if (st) return st;
+    if constexpr (std::is_same<T, float>::value) {
+        pack_corners_kernel<<<ceil_div(long(nrow), 256), 256>>>(
+            t->ntemp, t->npres, t->neta, t->ngpt, v.kmajor, t->planck_frac ? v.planck_frac : nullptr,
+            const_cast<float4*>(v.kmaj4), const_cast<float4*>(v.pfrac4), const_cast<Tab8*>(v.kmp8));
+        RB_LAUNCH("pack_corners_kernel");
+        RB_CUDA(cudaStreamSynchronize(nullptr), "pack_corners_kernel");   // the handle may be used on any stream
+    }
+    return RRTMGP_B200_OK;
 }
 
 }  // namespace
@@ -438,6 +475,7 @@ int rrtmgp_b200_kdist_create(const rrtmgp_b200_kdist_tables* t, const char* cons
         return st;
     };
     cudaGetDevice(&k->device);
+    cudaDeviceGetAttribute(&k->nsm, cudaDevAttrMultiProcessorCount, k->device);
 
     std::vector<std::string> names, avail;
     for (int i = 0; i < t->ngas; ++i) names.push_back(trim(t->gas_names[i]));
