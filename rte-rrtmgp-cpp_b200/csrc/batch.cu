@@ -75,6 +75,10 @@ struct TeamCtx {
     __device__ __forceinline__ int nloc(int nlay) const { return nlay; }
     template <class T>
     __device__ __forceinline__ void put(T* p, const T& v) const { *p = v; }
+    __device__ __forceinline__ int group0(int) const { return 0; }
+    __device__ __forceinline__ int group1(int ngroups) const { return ngroups; }
+    template <class... A>
+    __device__ __forceinline__ bool combine(A&...) const { return true; }
     __device__ __forceinline__ unsigned char* smem() const
     {
         extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -14,6 +14,14 @@ __global__ void __launch_bounds__(512) sw_forward_kernel(const KdistView<float> 
     sw_forward_column<CL, true, DENSE>(CtaCtx{}, k, io);
 }
 
+// Few columns: one thread-block cluster of `parts` CTAs per column, each a share of its g-points
+// (SplitCtx; xch: offset of its exchange buffer).
+template <int CL, bool DENSE>
+__global__ void __launch_bounds__(512) sw_forward_split_kernel(const KdistView<float> k, const SwGridIo io, int parts, int xch)
+{
+    sw_forward_column<CL, true, DENSE>(SplitCtx{parts, xch}, k, io);
+}
+
 // Columns of more than 16 chunks: one thread-block cluster of cs CTAs per column (ClusterCtx).
 template <int CL, bool DENSE>
 __global__ void __launch_bounds__(512) sw_forward_cluster_kernel(const KdistView<float> k, const SwGridIo io, int cs)
@@ -42,6 +50,9 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
         const cudaError_t e = cudaFuncSetAttribute(sw_forward_kernel<CL, DENSE>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
         if (e != cudaSuccess) return e;
+        const cudaError_t e2 = cudaFuncSetAttribute(sw_forward_split_kernel<CL, DENSE>,
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e2 != cudaSuccess) return e2;
         return cudaFuncSetAttribute(sw_forward_cluster_kernel<CL, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     220 * 1024);
     }, "forward_sw attribute");
@@ -55,23 +66,32 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
         ca.delta = delta;
     }
     SwGridIo io{ncol, nlay, play, plev, tlay, col_dry, mu0, tsi, alb_dir, alb_dif, up, dn, dir, net, hr, gs, ca, aer};
-    if (CS == 1) {
+    // the split's exchange buffer: 6 accumulators per thread
+    const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 6 * NW * 32;
+    const int parts = CS == 1 && split_smem <= 227 * 1024 ? group_parts(ncol, v.ngroups, NW * 32, split_smem, k->nsm) : 1;
+    if (CS == 1 && parts == 1) {
         sw_forward_kernel<CL, DENSE><<<ncol, NW * 32, smem, stream>>>(v, io);
         RB_LAUNCH("sw_forward_kernel");
         return RRTMGP_B200_OK;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(ncol) * CS);
+    const int cluster = CS == 1 ? parts : CS;
+    cfg.gridDim = dim3(unsigned(ncol) * cluster);
     cfg.blockDim = dim3(NWc * 32);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = CS == 1 ? split_smem : smem;
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = unsigned(CS);
+    at[0].val.clusterDim.x = unsigned(cluster);
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    if (CS == 1) {
+        RB_CUDA(cudaLaunchKernelEx(&cfg, sw_forward_split_kernel<CL, DENSE>, v, io, parts, int(xch)),
+                "sw_forward_split_kernel");
+        return RRTMGP_B200_OK;
+    }
     RB_CUDA(cudaLaunchKernelEx(&cfg, sw_forward_cluster_kernel<CL, DENSE>, v, io, CS), "sw_forward_cluster_kernel");
     return RRTMGP_B200_OK;
 }

@@ -11,6 +11,7 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -342,6 +343,10 @@ struct CtaCtx {
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     template <class T>
     __device__ __forceinline__ void put(T* p, const T& v) const { *p = v; }
+    __device__ __forceinline__ int group0(int) const { return 0; }
+    __device__ __forceinline__ int group1(int ngroups) const { return ngroups; }
+    template <class... A>
+    __device__ __forceinline__ bool combine(A&...) const { return true; }
 };
 
 // One column on a thread-block cluster of cs CTAs (columns deeper than one CTA holds): CTA r
@@ -376,7 +381,59 @@ struct ClusterCtx {
         cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
         for (int r = 0; r < cs; ++r) *cl.map_shared_rank(p, r) = v;
     }
+    __device__ __forceinline__ int group0(int) const { return 0; }
+    __device__ __forceinline__ int group1(int ngroups) const { return ngroups; }
+    template <class... A>
+    __device__ __forceinline__ bool combine(A&...) const { return true; }
 };
+
+// One column on a thread-block cluster of `parts` CTAs that share its g-points (grids of too few
+// columns to fill the chip): every CTA holds all layers and computes the groups [rank G / parts,
+// (rank + 1) G / parts); the FP64 accumulators are then added in rank order by CTA 0 through
+// distributed shared memory (xch: the byte offset of nthreads doubles per accumulator behind the
+// column's shared memory).
+struct SplitCtx : CtaCtx {
+    int parts, xch;
+    __device__ __forceinline__ SplitCtx(int p, int x) : parts(p), xch(x) {}
+    __device__ __forceinline__ int rank() const { return int(cooperative_groups::this_cluster().block_rank()); }
+    __device__ __forceinline__ int icol() const { return blockIdx.x / parts; }
+    __device__ __forceinline__ int group0(int ngroups) const { return rank() * ngroups / parts; }
+    __device__ __forceinline__ int group1(int ngroups) const { return (rank() + 1) * ngroups / parts; }
+    template <class... A>
+    __device__ __forceinline__ bool combine(A&... a) const
+    {
+        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        double* const own = reinterpret_cast<double*>(smem() + xch) + tid();
+        const int r = rank();
+        int i = 0;
+        if (r > 0) ((own[nthreads() * i++] = a), ...);
+        cl.sync();
+        if (r == 0)
+            for (int p = 1; p < parts; ++p) {
+                const double* const other = cl.map_shared_rank(own, p);
+                i = 0;
+                ((a += other[nthreads() * i++]), ...);
+            }
+        cl.sync();   // no CTA leaves while its shared memory may still be read
+        return r == 0;
+    }
+};
+
+// CTAs per column for a grid of ncol columns whose CTAs of `threads` threads (128 registers each)
+// and smem bytes, sharing the G groups of a column.  A CTA costs its groups and kGroupSetup more for its
+// set-up (layer state, scalings, cloud optics, launch); waves of CTAs run one after the other.
+// The split with the least waves x cost is taken when it saves more than a tenth.
+constexpr float kGroupSetup = 2.0f;   // measured 1.4 (LW) to 3 (SW) groups at 60 layers
+inline int group_parts(int ncol, int G, int threads, size_t smem, int nsm, int most = 8)
+{
+    const int per_sm = int(std::max<size_t>(1, std::min<size_t>(512 / threads, (227 * 1024) / (smem + 1024))));
+    const long slots = long(nsm) * per_sm;
+    auto cost = [&](int s) { return float((long(ncol) * s + slots - 1) / slots) * (kGroupSetup + float((G + s - 1) / s)); };
+    int best = 1;
+    for (int s = 2; s <= std::min(G, most); ++s)
+        if (cost(s) < 0.9f * cost(1) && cost(s) < cost(best)) best = s;
+    return best;
+}
 
 // Fill the per-layer state and col_gas of layers j0 .. j0 + nloc - 1 (counted from the top,
 // those below nlay) of column icol into st[j - j0] and cg[(gas) * cg_stride + j - j0]; threads

@@ -72,7 +72,7 @@ __device__ __forceinline__ void build_lw_record(const KdistView<float>& k, LwRec
 // sizes, arrays, gas set, cloud arrays) so that the batched kernel, which keeps them in shared
 // memory, holds no register for them across the column (see LwGridIo / CtaCtx for the per-grid
 // kernel, where they are launch constants).
-// PAIR (8-layer chunks): the records of groups gg and gg + 1 are built together at even gg
+// PAIR (8-layer chunks): the records of groups gg and gg + 1 are built together at every other gg
 // into two buffers (one group's 16 records per warp leave half the lanes idle).
 template <int CL, bool PAIR = false, bool DENSE = false, class Cx, class Io>
 __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<float>& k, const Io& io)
@@ -133,10 +133,12 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
     const int ngpt = k.ngpt;
     double acc_lev = 0.0, acc_div = 0.0, acc_bot_up = 0.0, acc_bot_dn = 0.0;
 
-    for (int gg = 0; gg < k.ngroups; ++gg) {
+    const int gbeg = cx.group0(k.ngroups), gend = cx.group1(k.ngroups);
+    for (int gg = gbeg; gg < gend; ++gg) {
+        const int par = (gg - gbeg) & 1;
         const int nlay = io.nlay();
-        float4* const sm_maps = sm_maps0 + (gg & 1) * cx.nwarps() * 32;
-        float* const sm_sfc = sm_sfc0 + (gg & 1) * 32;
+        float4* const sm_maps = sm_maps0 + par * cx.nwarps() * 32;
+        float* const sm_sfc = sm_sfc0 + par * 32;
         const int g = 32 * gg + lane;
         const bool gv = g < ngpt;
         const int b0 = k.group_band0[gg];
@@ -145,16 +147,16 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
         const MinorRef mr0 = minor_ref(k, 0, g, gv), mr1 = minor_ref(k, 1, g, gv);
 
         // 1. records of this warp's chunk
-        LwRec* const recs = recs0 + (P2 ? (gg & 1) : 0) * rbuf;
-        if (!P2 || (gg & 1) == 0) {
+        LwRec* const recs = recs0 + (P2 ? par : 0) * rbuf;
+        if (!P2 || par == 0) {
             const int nrec = CL * k.max_group_bands;
             for (int t = lane; t < (P2 ? 2 : 1) * nrec; t += 32) {
                 const int gq = gg + t / nrec, r = t % nrec;
-                if (gq >= k.ngroups) continue;
+                if (gq >= gend) continue;
                 const int jj = cx.warp() * CL + (r % CL), jl = jj - L0;
                 const int b = k.group_band0[gq] + r / CL;
                 if (jj < nlay && b < nband && k.band_lims[2 * b] < 32 * gq + 32)
-                    build_lw_record(k, recs0[(P2 ? (gq & 1) : 0) * rbuf + r], st[jl], sm_cg + jl, NL, b,
+                    build_lw_record(k, recs0[(gq - gg) * rbuf + r], st[jl], sm_cg + jl, NL, b,
                                     sm_cld[b * NL + jl], jj == nlay - 1, ts);
             }
         }
@@ -235,6 +237,8 @@ __device__ __forceinline__ void lw_forward_column(const Cx& cx, const KdistView<
             acc_bot_dn += double(warp_sum(rd));
         }
     }
+
+    if (!cx.combine(acc_lev, acc_div, acc_bot_up, acc_bot_dn)) return;
 
     // Outputs.  Fluxes = 2 pi w * (sum of radiances) with w = 0.5.
     const int w = cx.warp(), NW = cx.nwarps(), icol = cx.icol(), ncol = io.ncol(), nlay = io.nlay();

@@ -61,7 +61,7 @@ struct SwGridIo {
 // One column by the warps that context cx names (cx.nwarps() warps of CL layers each,
 // nlay <= cx.nwarps() * CL; chunks past nlay are identity layers).  Context and arguments are
 // read through accessors at every use, as in lw_forward_column.
-// PAIR (8-layer chunks): the records of groups gg and gg + 1 are built together at even gg
+// PAIR (8-layer chunks): the records of groups gg and gg + 1 are built together at every other gg
 // into two buffers (one group's 16 records per warp leave half the lanes idle).
 template <int CL, bool PAIR = false, bool DENSE = false, class Cx, class Io>
 __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<float>& k, const Io& io)
@@ -124,7 +124,9 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
     double acc_a = 0.0, acc_b = 0.0, acc_c = 0.0;   // see the output section
     double acc_sfc_dir = 0.0, acc_sfc_dn = 0.0, acc_sfc_up = 0.0;
 
-    for (int gg = 0; gg < k.ngroups; ++gg) {
+    const int gbeg = cx.group0(k.ngroups), gend = cx.group1(k.ngroups);
+    for (int gg = gbeg; gg < gend; ++gg) {
+        const int par = (gg - gbeg) & 1;
         const int nlay = io.nlay();
         const int g = 32 * gg + lane;
         const bool gv = g < ngpt;
@@ -133,17 +135,17 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
         const int slot = gband - b0;
         const MinorRef mr0 = minor_ref(k, 0, g, gv), mr1 = minor_ref(k, 1, g, gv);
 
-        SwRec* const recs = recs0 + (P2 ? (gg & 1) : 0) * rbuf;
-        if (!P2 || (gg & 1) == 0) {
+        SwRec* const recs = recs0 + (P2 ? par : 0) * rbuf;
+        if (!P2 || par == 0) {
             const int nrec = CL * k.max_group_bands;
             for (int t = lane; t < (P2 ? 2 : 1) * nrec; t += 32) {
                 const int gq = gg + t / nrec, r = t % nrec;
-                if (gq >= k.ngroups) continue;
+                if (gq >= gend) continue;
                 const int jj = cx.warp() * CL + (r % CL);
                 const int b = k.group_band0[gq] + r / CL;
                 if (jj < nlay && b < nband && k.band_lims[2 * b] < 32 * gq + 32) {
                     const int l = top_at_1 ? jj : nlay - 1 - jj;
-                    build_sw_record(k, recs0[(P2 ? (gq & 1) : 0) * rbuf + r], st[jj - L0], sm_cg + (jj - L0), NL, b,
+                    build_sw_record(k, recs0[(gq - gg) * rbuf + r], st[jj - L0], sm_cg + (jj - L0), NL, b,
                                     io.cloud(), cx.icol() + size_t(l) * io.ncol(),
                                     with_aer ? sm_aer + b * NL + (jj - L0) : nullptr);
                 }
@@ -320,6 +322,8 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
         acc_b += double(vUp[0]);
         acc_c += double(vDn[0]);
     }
+
+    if (!cx.combine(acc_a, acc_b, acc_c, acc_sfc_dir, acc_sfc_dn, acc_sfc_up)) return;
 
     // Outputs.  Lane L holds value v = L >> SH of the reduced arrays: v < CL is level
     // w*CL + v (acc_a: direct, acc_b: up, acc_c: diffuse down), v >= CL is layer

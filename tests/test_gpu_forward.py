@@ -236,3 +236,27 @@ def test_fused_deep_columns_on_clusters(oracle_mod, tables, gpu, nlay, top_at_1)
                                 oracle_mod.CloudOptics(tables["cloud_sw"]), atm)
     _check(lw, rlw, atm, f"deep lw nlay={nlay}")
     _check_sw(sw, rsw, f"deep sw nlay={nlay}")
+
+
+@pytest.mark.parametrize("nlay", [7, 60, 91, 128])   # one chunk, partial and full last chunks
+@pytest.mark.parametrize("ncol", [1, 45, 130])       # all, half and two parts of a column's groups per CTA
+def test_fused_forward_group_split(tables, gpu, ncol, nlay):
+    """Few columns share each column's g-points between the CTAs of a cluster; the same columns inside
+    a grid that fills the chip run unsplit.  The two differ only in the order of FP64 additions of
+    the groups' FP32 sums, so the FP32 outputs agree to the rounding of each (2 ulp), the
+    absorbed-flux sums and net fluxes to that of the terms they are differences of."""
+    import torch
+    from rrtmgp_b200.shard import slice_columns
+    from rrtmgp_b200.solver import atm_to_device
+    _, fused = _solvers(tables)
+    atm = S.make_atmosphere(2400, nlay, seed=70 + nlay, clouds=True)
+    _vary_surface(atm, 5)
+    part = slice_columns(atm, 0, ncol)
+    a, b = atm_to_device(atm, torch.float32, gpu), atm_to_device(part, torch.float32, gpu)
+    for solve in (fused.solve_lw, fused.solve_sw):
+        whole = {k: v[:, :ncol].clone() for k, v in solve(a).items()}
+        split = solve(b)
+        for k, w in whole.items():
+            scale = w.abs().clamp_min(1e-3 * float(w.abs().max()))
+            err = float(((split[k] - w).abs() / scale).max())
+            assert err < 5e-6, f"{solve.__name__} {k}: {err:.2e}"
