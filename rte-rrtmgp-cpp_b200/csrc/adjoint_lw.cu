@@ -151,21 +151,25 @@ __device__ __forceinline__ Tp* remote(cg::cluster_group& cl, Tp* p, int rank)
 // as NWc warps of CL layers; chunk maps and the surface source are pushed to every CTA of the
 // cluster through distributed shared memory.
 // DENSE: more than three minor intervals over some g-point (tau_abs).
-template <int CL, bool CLUSTER, bool FLUX, bool DENSE>
+// SPLIT (CLUSTER = false): few columns; a cluster of `parts` CTAs shares the groups of a column as
+// SplitCtx does in the forward kernel, CTA 0 adding the accumulators.
+template <int CL, bool CLUSTER, bool FLUX, bool DENSE, bool SPLIT = false>
 __global__ void __launch_bounds__(CL == 16 ? 256 : 512, 1)
 lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjCloud cld, int ncol, int nlay, int CS,
                   int idx_o3, int cd_internal, const float* __restrict__ play, const float* __restrict__ plev,
                   const float* __restrict__ tlay, const float* __restrict__ tlev, const float* __restrict__ tsfc,
                   const float* __restrict__ col_dry_in, const float* __restrict__ sfc_emis,
                   const float* __restrict__ seed_up, const float* __restrict__ seed_dn,
-                  const float* __restrict__ seed_hr, const AdjOut out)
+                  const float* __restrict__ seed_hr, const AdjOut out, int parts = 1)
 {
     static_assert(CL == 8 || CL == 16, "chunk length");
+    static_assert(!(SPLIT && CLUSTER), "a split column is one CTA deep");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cg::cluster_group cluster = cg::this_cluster();
     if (!CLUSTER) CS = 1;
     const int rank = CLUSTER ? int(cluster.block_rank()) : 0;
-    const int icol = blockIdx.x / CS;
+    const int part = SPLIT ? int(cluster.block_rank()) : 0;
+    const int icol = blockIdx.x / (SPLIT ? parts : CS);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int NWc = blockDim.x >> 5;       // warps of this CTA
     const int NWt = CS * NWc;               // chunks of the column
@@ -259,8 +263,9 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
     // divergences reduce-scattered over the group's g-points, the bottom level separately
     double acc_flev = 0.0, acc_fdiv = 0.0, acc_fbot_up = 0.0, acc_fbot_dn = 0.0;
 
-    for (int gg = 0; gg < k.ngroups; ++gg) {
-        const int pb = CLUSTER ? 0 : (gg & 1);
+    const int gbeg = SPLIT ? part * k.ngroups / parts : 0, gend = SPLIT ? (part + 1) * k.ngroups / parts : k.ngroups;
+    for (int gg = gbeg; gg < gend; ++gg) {
+        const int pb = CLUSTER ? 0 : ((gg - gbeg) & 1);
         float4* const sm_mapA = sm_map0 + pb * NWt * 32 * 2;                 // (A, Bd, Bu, BUbar) per chunk
         float* const sm_mapB = reinterpret_cast<float*>(sm_mapA + NWt * 32);  // BIbar per chunk
         float* const sm_sfc = sm_sfc0 + pb * 32;
@@ -505,6 +510,37 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
         if (CLUSTER) csync();   // maps and the surface source are rewritten by the next group
     }
 
+    if (SPLIT) {
+        // add the other CTAs' accumulators and cloud sums, in rank order; the records' space holds
+        // the exchange (32 doubles per warp and accumulator)
+        __syncthreads();
+        double* const own = reinterpret_cast<double*>(smem_raw + SL.recs) + threadIdx.x;
+        auto each = [&](auto&& f) {
+            int i = 0;
+#pragma unroll
+            for (int r = 0; r < NRS; ++r) f(acc[r], i++);
+            f(acc_levbot, i++);
+            f(acc_tsfc, i++);
+            if (FLUX) {
+                f(acc_flev, i++);
+                f(acc_fdiv, i++);
+                f(acc_fbot_up, i++);
+                f(acc_fbot_dn, i++);
+            }
+        };
+        if (part > 0) each([&](double& a, int i) { own[i * int(blockDim.x)] = a; });
+        cluster.sync();
+        if (part == 0)
+            for (int p = 1; p < parts; ++p) {
+                const double* const other = remote(cluster, own, p);
+                each([&](double& a, int i) { a += other[i * int(blockDim.x)]; });
+                const float* const tb = remote(cluster, sm_tb, p);
+                for (int i = threadIdx.x; i < LPC * nband; i += blockDim.x) sm_tb[i] += tb[i];
+            }
+        cluster.sync();   // no CTA leaves while its shared memory may still be read
+        if (part > 0) return;
+    }
+
     // ---- outputs ----
     if (FLUX) {
         constexpr int SH_LEV = (CL == 16) ? 0 : 1;   // lane L holds value L >> SH_LEV
@@ -622,6 +658,9 @@ int launch_lw_adjoint(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
         const cudaError_t e = cudaFuncSetAttribute(lw_adjoint_kernel<CL, false, FLUX, DENSE>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
+        const cudaError_t e2 = cudaFuncSetAttribute(lw_adjoint_kernel<8, false, FLUX, DENSE, true>,
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e2 != cudaSuccess) return e2;
         return cudaFuncSetAttribute(lw_adjoint_kernel<8, true, FLUX, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024);
     }, "adjoint_lw attribute");
@@ -633,27 +672,35 @@ int launch_lw_adjoint(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
         ca.lwp = lwp; ca.iwp = iwp; ca.rel = rel; ca.rei = rei;
         ca.present = 1;
     }
-    if (CS == 1) {
+    const int parts = CS == 1 && CL == 8 ? group_parts(ncol, v.ngroups, NWc * 32, smem, k->nsm) : 1;
+    if (CS == 1 && parts == 1) {
         lw_adjoint_kernel<CL, false, FLUX, DENSE><<<ncol, NWc * 32, smem, stream>>>(v, gs, ca, ncol, nlay, 1, idx_o3, col_dry ? 0 : 1,
                                                                   play, plev, tlay, tlev, tsfc, col_dry, emis, su, sd,
-                                                                  sh, out);
+                                                                  sh, out, 1);
         RB_LAUNCH("lw_adjoint_kernel");
         return RRTMGP_B200_OK;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(ncol) * CS);
+    const int cluster = CS == 1 ? parts : CS;
+    cfg.gridDim = dim3(unsigned(ncol) * cluster);
     cfg.blockDim = dim3(NWc * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = unsigned(CS);
+    at[0].val.clusterDim.x = unsigned(cluster);
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    if (CS == 1) {
+        RB_CUDA(cudaLaunchKernelEx(&cfg, lw_adjoint_kernel<8, false, FLUX, DENSE, true>, v, gs, ca, ncol, nlay, 1, idx_o3,
+                                   col_dry ? 0 : 1, play, plev, tlay, tlev, tsfc, col_dry, emis, su, sd, sh, out, parts),
+                "lw_adjoint_kernel split launch");
+        return RRTMGP_B200_OK;
+    }
     RB_CUDA(cudaLaunchKernelEx(&cfg, lw_adjoint_kernel<8, true, FLUX, DENSE>, v, gs, ca, ncol, nlay, CS, idx_o3, col_dry ? 0 : 1, play,
-                               plev, tlay, tlev, tsfc, col_dry, emis, su, sd, sh, out),
+                               plev, tlay, tlev, tsfc, col_dry, emis, su, sd, sh, out, 1),
             "lw_adjoint_kernel launch");
     return RRTMGP_B200_OK;
 }

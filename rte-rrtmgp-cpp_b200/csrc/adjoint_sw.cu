@@ -27,6 +27,8 @@
 // gas/Rayleigh/cloud combination, and the gas-optics interpolation (adjoint_common.cuh).
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "adjoint_common.cuh"
 #include "dual.cuh"
 #include "sw_common.cuh"
@@ -476,7 +478,10 @@ __device__ __forceinline__ Tp* remote(cg::cluster_group& cl, Tp* p, int rank)
 // CL layers per warp, kLPC / CL warps per CTA: CL = 8 gives 8 warps with up to 255 registers,
 // CL = 4 gives 16 warps at 128 registers (half the per-layer values per thread).
 // DENSE: more than three minor intervals over some g-point (sw_layer_forward/adjoint).
-template <int CL, bool FLUX, bool PAIR, bool DENSE>
+// SPLIT: few columns; the cluster has `parts` times CS CTAs, part p computing a share of the column's
+// groups on the CS CTAs [p CS, (p + 1) CS), whose sums part 0 adds at the end.  Every part runs
+// the same number of groups (the cluster barrier is all parts'), the last ones with no valid g-point.
+template <int CL, bool FLUX, bool PAIR, bool DENSE, bool SPLIT>
 __global__ void __launch_bounds__(kLPC / CL * 32, 1)
 sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwCloudArgs cld, int ncol, int nlay, int CS,
                   int idx_o3, int cd_internal, const float* __restrict__ play, const float* __restrict__ plev,
@@ -485,13 +490,15 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
                   const float* __restrict__ alb_dir, const float* __restrict__ alb_dif,
                   const float* __restrict__ seed_up, const float* __restrict__ seed_dn,
                   const float* __restrict__ seed_dir, const float* __restrict__ seed_hr, const SwAdjOut out,
-                  const SwAerosolArgs aer)
+                  const SwAerosolArgs aer, int parts)
 {
     constexpr int WPC = kLPC / CL;   // warps per CTA
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = int(cluster.block_rank());
-    const int icol = blockIdx.x / CS;
+    const int part = SPLIT ? int(cluster.block_rank()) / CS : 0;
+    const int rank = int(cluster.block_rank()) - part * CS;   // within the part
+    const int icol = blockIdx.x / (SPLIT ? parts * CS : CS);
+    const int rr0 = part * CS;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int Wg = rank * WPC + w;
     const int NWt = CS * WPC;
@@ -590,10 +597,13 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
     double acc_sfc_dir = 0.0, acc_sfc_dn = 0.0, acc_sfc_up = 0.0;
     constexpr float m_dry = 0.028964f, m_h2o = 0.018016f;
 
-    for (int gg = 0; gg < k.ngroups; ++gg) {
+    const int gper = SPLIT ? (k.ngroups + parts - 1) / parts : k.ngroups;
+    const int gbeg = SPLIT ? part * gper : 0, gend = SPLIT ? min(k.ngroups, gbeg + gper) : k.ngroups;
+    for (int gg = gbeg; gg < gbeg + gper; ++gg) {
+        const int par = (gg - gbeg) & 1;
         const int g = 32 * gg + lane;
-        const bool gv = g < ngpt;
-        const int b0 = k.group_band0[gg];
+        const bool gv = g < ngpt && (!SPLIT || gg < gend);
+        const int b0 = k.group_band0[SPLIT ? min(gg, k.ngroups - 1) : gg];
         const int gband = gv ? k.gpt2band[g] : b0;
         const int slot = gband - b0;
         const MinorRef mr0 = minor_ref(k, 0, g, gv), mr1 = minor_ref(k, 1, g, gv);
@@ -604,18 +614,18 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
         // records of groups gg and gg + 1 are built together at even gg into two buffers: with
         // 8 layers and 2 bands a group has 16 records per warp, so one group alone leaves half
         // the lanes idle.
-        SwRec* const recs = recs0 + (PAIR ? (gg & 1) : 0) * kLPC * mgb;
-        DRec* const drecs = drecs0 + (PAIR ? (gg & 1) : 0) * kLPC * mgb;
-        if (!PAIR || (gg & 1) == 0) {
+        SwRec* const recs = recs0 + (PAIR ? par : 0) * kLPC * mgb;
+        DRec* const drecs = drecs0 + (PAIR ? par : 0) * kLPC * mgb;
+        if (!PAIR || par == 0) {
             const int nrec = CL * mgb;
             for (int t = lane; t < (PAIR ? 2 : 1) * nrec; t += 32) {
                 const int gq = gg + t / nrec, r = t % nrec;
-                if (gq >= k.ngroups) continue;
+                if (gq >= gend) continue;
                 const int jl = w * CL + (r % CL);
                 const int jj = j0 + jl;
                 const int b = k.group_band0[gq] + r / CL;
                 if (jj < nlay && b < nband && k.band_lims[2 * b] < 32 * gq + 32) {
-                    const int qb = PAIR ? (gq & 1) : 0;
+                    const int qb = gq - gg;
                     const int l = top_at_1 ? jj : nlay - 1 - jj;
                     const LayerState s = st[jl];
                     build_sw_record(k, recs0[qb * kLPC * mgb + r], s, sm_cg + jl, kLPC, b, cld, icol + size_t(l) * ncol,
@@ -663,7 +673,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             cRu = nRu; cRd = nRd; cU = nU; cD = nD;
             P *= Tn;
         }
-        for (int rr = 0; rr < CS; ++rr) remote(cluster, sm_x1, rr)[Wg * 32 + lane] = P;
+        for (int rr = rr0; rr < rr0 + CS; ++rr) remote(cluster, sm_x1, rr)[Wg * 32 + lane] = P;
         cluster.sync();
 
         // ---- X1: direct flux at the chunk top and the surface ----
@@ -672,7 +682,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
         for (int c = 0; c < Wg; ++c) dtop *= sm_x1[c * 32 + lane];
         float dsfc = dtop;
         for (int c = Wg; c < NWt; ++c) dsfc *= sm_x1[c * 32 + lane];
-        for (int rr = 0; rr < CS; ++rr) {
+        for (int rr = rr0; rr < rr0 + CS; ++rr) {
             remote(cluster, sm_x2a, rr)[Wg * 32 + lane] = make_float4(cRu, cRd, cT, cU * dtop);
             remote(cluster, sm_x2b, rr)[Wg * 32 + lane] = cD * dtop;
         }
@@ -780,7 +790,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
                 A3 *= c;
                 B3 = c * B3 + off;
             }
-            for (int rr = 0; rr < CS; ++rr) remote(cluster, sm_x3, rr)[Wg * 32 + lane] = make_float2(A3, B3);
+            for (int rr = rr0; rr < rr0 + CS; ++rr) remote(cluster, sm_x3, rr)[Wg * 32 + lane] = make_float2(A3, B3);
         }
         cluster.sync();
         float Fraw = (L_end == nlay) ? beN + alN * af : 0.f;
@@ -819,7 +829,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
                 const float nR = r * cR, nV = r * cV + v;
                 cP = nP; cQ = nQ; cUo = nU; cR = nR; cV = nV;
             }
-            for (int rr = 0; rr < CS; ++rr) {
+            for (int rr = rr0; rr < rr0 + CS; ++rr) {
                 remote(cluster, sm_x4a, rr)[Wg * 32 + lane] = make_float4(cP, cQ, cR, cUo);
                 remote(cluster, sm_x4b, rr)[Wg * 32 + lane] = cV;
             }
@@ -887,7 +897,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
                 A5 *= vTn[i];
                 B5 = vTn[i] * B5 + e;
             }
-            for (int rr = 0; rr < CS; ++rr) remote(cluster, sm_x5, rr)[Wg * 32 + lane] = make_float2(A5, B5);
+            for (int rr = rr0; rr < rr0 + CS; ++rr) remote(cluster, sm_x5, rr)[Wg * 32 + lane] = make_float2(A5, B5);
         }
         cluster.sync();
         float Db = SbN * ad + ((L_end == nlay) ? beN + gaN : 0.f);
@@ -965,6 +975,37 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
         // and 256 layers.)
     }
 
+    if (SPLIT) {
+        // part 0 adds the other parts' accumulators, cloud and albedo sums, in part order; the records'
+        // space holds the exchange (32 doubles per warp and accumulator)
+        __syncthreads();
+        double* const own = reinterpret_cast<double*>(smem_raw + SL.recs) + threadIdx.x;
+        auto each = [&](auto&& f) {
+            f(acc_q, 0);
+            if (FLUX) {
+                f(acc_fa, 1);
+                f(acc_fb, 2);
+                f(acc_fc, 3);
+                f(acc_sfc_dir, 4);
+                f(acc_sfc_dn, 5);
+                f(acc_sfc_up, 6);
+            }
+        };
+        if (part > 0) each([&](double& a, int i) { own[i * int(blockDim.x)] = a; });
+        cluster.sync();
+        if (part == 0)
+            for (int p = 1; p < parts; ++p) {
+                const double* const other = remote(cluster, own, p * CS + rank);
+                each([&](double& a, int i) { a += other[i * int(blockDim.x)]; });
+                const float* const cl = remote(cluster, sm_cl, p * CS + rank);
+                for (int i = threadIdx.x; i < nband * kLPC * 3; i += blockDim.x) sm_cl[i] += cl[i];
+                const double* const al = remote(cluster, sm_alb, p * CS + rank);
+                for (int i = threadIdx.x; i < nband * 2; i += blockDim.x) sm_alb[i] += al[i];
+            }
+        cluster.sync();   // no CTA leaves while its shared memory may still be read
+        if (part > 0) return;
+    }
+
     // ---- outputs ----
     __syncthreads();   // the cloud sums of the last group are read below by other warps
     if (FLUX) {
@@ -1039,7 +1080,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
             if (out.alb_dif) out.alb_dif[b + size_t(icol) * nband] = float(sm_alb[2 * b + 1]);
         }
     }
-    cluster.sync();   // no CTA leaves while its shared memory may still be read remotely
+    if (!SPLIT) cluster.sync();   // no CTA leaves while its shared memory may still be read remotely
 }
 
 }  // namespace
@@ -1098,10 +1139,13 @@ int adjoint_sw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay,
     if (smem > 227 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "adjoint_sw: shared memory need exceeds 227 KB");
     static PerDeviceOnce attr;
     const int ast = attr.run([] {
-        for (auto fn : {sw_adjoint_kernel<CL, false, false, false>, sw_adjoint_kernel<CL, true, false, false>,
-                        sw_adjoint_kernel<CL, false, true, false>, sw_adjoint_kernel<CL, true, true, false>,
-                        sw_adjoint_kernel<CL, false, false, true>, sw_adjoint_kernel<CL, true, false, true>,
-                        sw_adjoint_kernel<CL, false, true, true>, sw_adjoint_kernel<CL, true, true, true>}) {
+        for (auto fn :
+             {sw_adjoint_kernel<CL, false, false, false, false>, sw_adjoint_kernel<CL, true, false, false, false>,
+              sw_adjoint_kernel<CL, false, true, false, false>, sw_adjoint_kernel<CL, true, true, false, false>,
+              sw_adjoint_kernel<CL, false, false, true, false>, sw_adjoint_kernel<CL, true, false, true, false>,
+              sw_adjoint_kernel<CL, false, true, true, false>, sw_adjoint_kernel<CL, true, true, true, false>,
+              sw_adjoint_kernel<CL, false, true, false, true>, sw_adjoint_kernel<CL, true, true, false, true>,
+              sw_adjoint_kernel<CL, false, true, true, true>, sw_adjoint_kernel<CL, true, true, true, true>}) {
             const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (e != cudaSuccess) return e;
         }
@@ -1118,28 +1162,32 @@ int adjoint_sw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay,
     }
     const SwAdjOut out{g_tlay, g_h2o, g_o3, g_lwp, g_iwp, g_rel, g_rei, g_alb_dir, g_alb_dif,
                        flux_up, flux_dn, flux_dir, flux_net, heating_rate};
+    // parts of a column's groups per cluster: one CTA of this kernel per SM (255 registers), at most
+    // 8 CTAs in a cluster
+    const int parts = pair && 2 * CS <= 8 ? group_parts(ncol * CS, v.ngroups, 512, smem, k->nsm, 8 / CS) : 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(ncol) * CS);
+    cfg.gridDim = dim3(unsigned(ncol) * CS * parts);
     cfg.blockDim = dim3(kLPC / CL * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = as_stream(stream);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = unsigned(CS);
+    at[0].val.clusterDim.x = unsigned(CS * parts);
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     const bool dense = v.max_minor_per_g > 3;
-    const auto kernel =
-        dense ? (with_flux ? (pair ? sw_adjoint_kernel<CL, true, true, true> : sw_adjoint_kernel<CL, true, false, true>)
-                           : (pair ? sw_adjoint_kernel<CL, false, true, true> : sw_adjoint_kernel<CL, false, false, true>))
-              : (with_flux ? (pair ? sw_adjoint_kernel<CL, true, true, false> : sw_adjoint_kernel<CL, true, false, false>)
-                           : (pair ? sw_adjoint_kernel<CL, false, true, false>
-                                   : sw_adjoint_kernel<CL, false, false, false>));
+    auto pick = [&](auto d) {
+        constexpr bool D = decltype(d)::value;
+        if (parts > 1) return with_flux ? sw_adjoint_kernel<CL, true, true, D, true> : sw_adjoint_kernel<CL, false, true, D, true>;
+        if (pair) return with_flux ? sw_adjoint_kernel<CL, true, true, D, false> : sw_adjoint_kernel<CL, false, true, D, false>;
+        return with_flux ? sw_adjoint_kernel<CL, true, false, D, false> : sw_adjoint_kernel<CL, false, false, D, false>;
+    };
+    const auto kernel = dense ? pick(std::true_type{}) : pick(std::false_type{});
     RB_CUDA(cudaLaunchKernelEx(&cfg, kernel, v, gs, ca, ncol, nlay, CS, idx_o3, col_dry ? 0 : 1, play, plev,
                                tlay, col_dry, mu0, tsi_scaling, sfc_alb_dir, sfc_alb_dif, seed_up, seed_dn, seed_dir,
-                               seed_hr, out, aer),
+                               seed_hr, out, aer, parts),
             "sw_adjoint_kernel launch");
     return RRTMGP_B200_OK;
 }

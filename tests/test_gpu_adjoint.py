@@ -353,3 +353,37 @@ def test_forward_adjoint_one_launch(tables, gpu, nlay):
             scale = float(ref_g[k].abs().max()) + 1e-30
             d = float((gr[k] - ref_g[k]).abs().max()) / scale
             assert d < 1e-4, f"{dom} grad {k}: {d:.3e}"
+
+
+@pytest.mark.parametrize("nlay", [7, 60, 80, 130])   # SW clusters of one, two and three CTAs deep; 130: LW unsplit
+@pytest.mark.parametrize("ncol", [1, 40])
+def test_adjoint_group_split(tables, gpu, ncol, nlay):
+    """Few columns share each column's g-points between the CTAs of a cluster; inside a grid that fills
+    the chip the same columns run unsplit, in another instance of the kernel.  Bound: each
+    instance's FP32 gradients are within 3.5e-4 of FP64 on the scale max(|value|, rms) (the o3
+    gradient, whose interpolation weights cancel by up to (2 neta - 1) terms; the others and the
+    fluxes are below 1e-5), so two instances differ by at most twice that; a group lost or
+    counted twice shows as a tenth or more."""
+    import torch
+    from rrtmgp_b200 import autodiff
+    from rrtmgp_b200.shard import slice_columns
+    from rrtmgp_b200.solver import Fused_solver, Radiation_solver, atm_to_device
+    base = Radiation_solver(tables["lw"], tables["sw"], tables["cloud_lw"], tables["cloud_sw"], S.ATM_GASES)
+    fused = Fused_solver(base)
+    atm = S.make_atmosphere(2400, nlay, seed=31 + nlay, clouds=True)
+    a = atm_to_device(atm, torch.float32, gpu)
+    b = atm_to_device(slice_columns(atm, 0, ncol), torch.float32, gpu)
+    gen = torch.Generator(device=gpu).manual_seed(3)
+    seeds = [torch.randn((nlay + n, 2400), generator=gen, device=gpu) for n in (1, 1, 1, 0)]
+    part = [s[:, :ncol].contiguous() for s in seeds]
+    for name, whole, split in (
+            ("lw", autodiff.adjoint_lw(fused, a, *(seeds[i] for i in (0, 1, 3)), with_fluxes=True),
+             autodiff.adjoint_lw(fused, b, *(part[i] for i in (0, 1, 3)), with_fluxes=True)),
+            ("sw", autodiff.adjoint_sw(fused, a, *seeds, with_fluxes=True),
+             autodiff.adjoint_sw(fused, b, *part, with_fluxes=True))):
+        for w, s in zip(whole, split):
+            for k in w:
+                ref = w[k][:ncol] if k.startswith("sfc_alb") or w[k].dim() == 1 else w[k][:, :ncol]
+                scale = ref.abs().clamp_min(float(ref.double().square().mean().sqrt()) + 1e-30)
+                err = float(((s[k] - ref).abs() / scale).max())
+                assert err < (7e-4 if k == "o3" else 2e-5), f"{name} {k}: {err:.2e}"
