@@ -8,8 +8,8 @@ namespace {
 using namespace fused;
 
 // DENSE: tables with more than three minor intervals over some g-point (tau_abs).
-template <int CL, bool DENSE>
-__global__ void __launch_bounds__(512) lw_forward_kernel(const KdistView<float> k, const LwGridIo io)
+template <int CL, bool DENSE, int THREADS = 512, int PER_SM = 1>
+__global__ void __launch_bounds__(THREADS, PER_SM) lw_forward_kernel(const KdistView<float> k, const LwGridIo io)
 {
     lw_forward_column<CL, true, DENSE>(CtaCtx{}, k, io);
 }
@@ -30,6 +30,20 @@ __global__ void __launch_bounds__(512) lw_forward_cluster_kernel(const KdistView
     cooperative_groups::this_cluster().sync();   // no CTA leaves while another may store into its shared memory
 }
 
+// The instance for columns of NW chunks of 8 layers: register caps that let more CTAs share an SM, as
+// the kernel waits on table loads (16 warps per SM at 128 registers).  At 80 registers (40 bytes
+// of spill loads) an SM holds 24 warps; 9 and 10 chunks need none at 96.
+template <int CL, bool DENSE>
+auto pick_forward(int NW) -> void (*)(const KdistView<float>, const LwGridIo)
+{
+    if constexpr (CL == 8) {
+        if (NW <= 8) return lw_forward_kernel<CL, DENSE, 256, 3>;
+        if (NW <= 10) return lw_forward_kernel<CL, DENSE, 320, 2>;
+        if (NW <= 12) return lw_forward_kernel<CL, DENSE, 384, 2>;
+    }
+    return lw_forward_kernel<CL, DENSE>;
+}
+
 template <int CL, bool DENSE>
 int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay, const float* play,
                       const float* plev, const float* tlay, const float* tlev, const float* tsfc, const float* col_dry,
@@ -46,9 +60,11 @@ int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_lw: shared memory need exceeds 220 KB");
     static PerDeviceOnce attr;
     int st = attr.run([] {
-        const cudaError_t e = cudaFuncSetAttribute(lw_forward_kernel<CL, DENSE>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return e;
+        for (int nw : {8, 10, 12, 16}) {   // every instance
+            const cudaError_t e = cudaFuncSetAttribute(pick_forward<CL, DENSE>(nw),
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+            if (e != cudaSuccess) return e;
+        }
         const cudaError_t e2 = cudaFuncSetAttribute(lw_forward_split_kernel<CL, DENSE>,
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e2 != cudaSuccess) return e2;
@@ -68,7 +84,7 @@ int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 4 * NW * 32;
     const int parts = CS == 1 && split_smem <= 227 * 1024 ? group_parts(ncol, v.ngroups, NW * 32, split_smem, k->nsm) : 1;
     if (CS == 1 && parts == 1) {
-        lw_forward_kernel<CL, DENSE><<<ncol, NW * 32, smem, stream>>>(v, io);
+        pick_forward<CL, DENSE>(NW)<<<ncol, NW * 32, smem, stream>>>(v, io);
         RB_LAUNCH("lw_forward_kernel");
         return RRTMGP_B200_OK;
     }
@@ -120,7 +136,10 @@ int forward_lw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay,
 #define RB_LW_FWD(CLv, D)                                                                                          \
     launch_lw_forward<CLv, D>(k, c, ncol, nlay, play, plev, tlay, tlev, tsfc, col_dry, gs, lwp, iwp, rel, rei, \
                               sfc_emis, flux_up, flux_dn, flux_net, heating_rate, s)
-    if (chunk == 8) return dense ? RB_LW_FWD(8, true) : RB_LW_FWD(8, false);
+    // Up to 12 chunks of 8 layers the 8-layer instances fit 18 - 25 warps per SM (pick_forward):
+    // 1000 x 72 274 -> 244 us, 4096 x 91 1.26 -> 1.12 ms, dense tables 2000 x 60 626 -> 547 us.  Deeper
+    // columns are faster in 16-layer chunks (8192 x 128: 2.93 ms, 3.24 - 3.5 with 8).
+    if (chunk ? chunk == 8 : nlay <= 96) return dense ? RB_LW_FWD(8, true) : RB_LW_FWD(8, false);
     return dense ? RB_LW_FWD(16, true) : RB_LW_FWD(16, false);
 #undef RB_LW_FWD
 }

@@ -8,8 +8,8 @@ namespace {
 using namespace fused;
 
 // DENSE: tables with more than three minor intervals over some g-point (tau_abs).
-template <int CL, bool DENSE>
-__global__ void __launch_bounds__(512) sw_forward_kernel(const KdistView<float> k, const SwGridIo io)
+template <int CL, bool DENSE, int THREADS = 512, int PER_SM = 1>
+__global__ void __launch_bounds__(THREADS, PER_SM) sw_forward_kernel(const KdistView<float> k, const SwGridIo io)
 {
     sw_forward_column<CL, true, DENSE>(CtaCtx{}, k, io);
 }
@@ -30,6 +30,25 @@ __global__ void __launch_bounds__(512) sw_forward_cluster_kernel(const KdistView
     cooperative_groups::this_cluster().sync();   // no CTA leaves while another may store into its shared memory
 }
 
+// The instance for columns of NW chunks.  The kernel waits on table loads, dependent arithmetic and the
+// chunk exchange, so more resident warps are worth some spills: at 128 registers an SM holds 16
+// warps, and 9 or 12 chunks leave a CTA alone on it.  At 96 registers (132 bytes of spill
+// loads) two CTAs of 9 or 10 chunks fit; at 80 (260) two of 11 or 12; at 64 (384) two of 13 - 16.
+// Measured against 128 registers: 1000 x 72 419 -> 313 us, 4096 x 91 1.72 -> 1.37 ms, 8192 x 128
+// 3.88 -> 3.57 ms.  Up to 8 chunks, where 15 or 16 warps fit at 128, the caps gained nothing (2000 x 60
+// 453 us, 461 at 80 registers; 2000 x 40 325 us, 324 at 96).
+template <int CL, bool DENSE>
+auto pick_forward(int NW) -> void (*)(const KdistView<float>, const SwGridIo)
+{
+    if constexpr (CL == 8) {
+        if (NW <= 8) return sw_forward_kernel<CL, DENSE>;
+        if (NW <= 10) return sw_forward_kernel<CL, DENSE, 320, 2>;
+        if (NW <= 12) return sw_forward_kernel<CL, DENSE, 384, 2>;
+        return sw_forward_kernel<CL, DENSE, 512, 2>;
+    }
+    return sw_forward_kernel<CL, DENSE>;
+}
+
 template <int CL, bool DENSE>
 int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay, const float* play,
                       const float* plev, const float* tlay, const float* col_dry, const GasSet<float>& gs,
@@ -47,9 +66,11 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_sw: shared memory need exceeds 220 KB");
     static PerDeviceOnce attr;
     int st = attr.run([] {
-        const cudaError_t e = cudaFuncSetAttribute(sw_forward_kernel<CL, DENSE>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return e;
+        for (int nw : {8, 10, 12, 16}) {   // every instance
+            const cudaError_t e = cudaFuncSetAttribute(pick_forward<CL, DENSE>(nw),
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+            if (e != cudaSuccess) return e;
+        }
         const cudaError_t e2 = cudaFuncSetAttribute(sw_forward_split_kernel<CL, DENSE>,
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e2 != cudaSuccess) return e2;
@@ -70,7 +91,7 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 6 * NW * 32;
     const int parts = CS == 1 && split_smem <= 227 * 1024 ? group_parts(ncol, v.ngroups, NW * 32, split_smem, k->nsm) : 1;
     if (CS == 1 && parts == 1) {
-        sw_forward_kernel<CL, DENSE><<<ncol, NW * 32, smem, stream>>>(v, io);
+        pick_forward<CL, DENSE>(NW)<<<ncol, NW * 32, smem, stream>>>(v, io);
         RB_LAUNCH("sw_forward_kernel");
         return RRTMGP_B200_OK;
     }
