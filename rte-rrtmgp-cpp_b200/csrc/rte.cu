@@ -1,6 +1,6 @@
 // Per-stage RTE solvers: longwave no-scattering (Gauss quadrature) and shortwave two-stream
 // with adding, over the reference's column-fastest (ncol, nlay|nlev, ngpt) arrays.
-//   * Up to 256 layers (one angle for the longwave; FP64 shortwave up to 128): the chunked
+//   * Up to 256 layers (longwave with several angles: FP32 up to 128; FP64 shortwave up to 128): the chunked
 //     kernels below -- a warp is 32 consecutive columns x a chunk of layers at one g-point,
 //     the chunks of a column are the warps of a block and exchange affine maps through shared
 //     memory -- read every input once and write every level once (no workspace, no stash).
@@ -216,13 +216,12 @@ struct LwChunkArgs {
 
 // Layer inputs (tau, Planck sources; tr/sdn/sup are overwritten with the transmissivity and
 // the layer sources) -> the chunk's maps: the down sweep x -> A x + Bd and the up sweep
-// x -> A x + Bu, stored at [w][lane] of sm_a, sm_bd, sm_bu.  One angle (D = 1.66, weight 0.5:
-// Rte_lw.cpp:101-113).
+// x -> A x + Bu, stored at [w][lane] of sm_a, sm_bd, sm_bu.  D: the secant (1.66, weight 0.5 with
+// one angle: Rte_lw.cpp:101-113).
 template <typename T, int CL>
 __device__ __forceinline__ void lw_chunk_maps(T (&tr)[CL], const T (&lay)[CL], T (&sdn)[CL], T (&sup)[CL], T* sm_a,
-                                              T* sm_bd, T* sm_bu, int w, int lane)
+                                              T* sm_bd, T* sm_bu, int w, int lane, T D = T(1.66))
 {
-    const T D = T(1.66);
     T A = T(1), Bd = T(0), Bu = T(0);
 #pragma unroll
     for (int i = 0; i < CL; ++i) {
@@ -245,10 +244,10 @@ __device__ __forceinline__ void lw_chunk_maps(T (&tr)[CL], const T (&lay)[CL], T
 // warp scanning the chunks above and below itself, the scans were O(chunks^2) loads per tile.
 template <typename T>
 __device__ __forceinline__ void lw_chunk_scan(const LwChunkArgs<T>& a, T* sm_a, T* sm_bd, T* sm_bu, int nw, int lane,
-                                              int ic, int g)
+                                              int ic, int g, T two_pi_w = pi_value<T>())
 {
     const int ncol = a.ncol;
-    T x = (a.inc_flux ? a.inc_flux[ic + size_t(g) * ncol] : T(0)) / pi_value<T>();
+    T x = (a.inc_flux ? a.inc_flux[ic + size_t(g) * ncol] : T(0)) / two_pi_w;
     for (int c = 0; c < nw; ++c) {
         const T A = sm_a[c * 32 + lane], B = sm_bd[c * 32 + lane];
         sm_bd[c * 32 + lane] = x;
@@ -347,6 +346,93 @@ __global__ void __launch_bounds__(MAXT) lw_solver_chunked(const LwChunkArgs<T> a
     __syncthreads();
     if (!cv) return;
     lw_chunk_levels<T, CL>(a, tr, sdn, sup, sm_a, sm_bd, sm_bu, w, lane, ic, g);
+}
+
+// Several quadrature angles in FP32, 8-layer chunks (nlay <= 128): as lw_solver_chunked, with the
+// layer inputs kept in registers over the angles and the levels' sums written once.  One thread per
+// (column, g-point) walking all layers of every angle, re-reading the inputs and adding to the
+// fluxes in memory, left a 500 x 60 grid at 7 warps per SM: three angles 368 -> 106 us (by the
+// difference of the whole call).
+// JAC: also the surface-temperature Jacobian.
+template <bool JAC>
+__global__ void __launch_bounds__(512) lw_solver_angles(const LwChunkArgs<float> a, int nmus,
+                                                        const float* __restrict__ tau, const float* __restrict__ lay_src,
+                                                        const float* __restrict__ lev_inc,
+                                                        const float* __restrict__ lev_dec)
+{
+    constexpr int CL = 8;
+    __shared__ float sm_a[16 * 32], sm_bd[16 * 32], sm_bu[16 * 32];   // chunk maps [chunk][lane]
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int ncol = a.ncol, nlay = a.nlay;
+    const int icol = blockIdx.x * 32 + lane;
+    const bool cv = icol < ncol;
+    const int ic = cv ? icol : 0;
+    const int g = blockIdx.y;
+    const size_t ncl = size_t(ncol) * nlay, ncv = size_t(ncol) * (nlay + 1);
+    const float* lev_dn = a.top_at_1 ? lev_inc : lev_dec;
+    const float* lev_up = a.top_at_1 ? lev_dec : lev_inc;
+    const int j0 = w * CL;
+    float vt[CL], vl[CL], vd[CL], vu[CL];
+#pragma unroll
+    for (int i = 0; i < CL; ++i) {
+        const int j = j0 + i;
+        vt[i] = 0.f; vl[i] = 0.f; vd[i] = 0.f; vu[i] = 0.f;
+        if (cv && j < nlay) {
+            const size_t x = ic + size_t(g) * ncl + size_t(a.top_at_1 ? j : nlay - 1 - j) * ncol;
+            vt[i] = tau[x];
+            vl[i] = lay_src[x];
+            vd[i] = lev_dn[x];
+            vu[i] = lev_up[x];
+        }
+    }
+    // sums over the angles: down at the level below and up at the level above each layer; the top
+    // level's down and the surface's up
+    float fdn[CL], fup[CL], fj[JAC ? CL : 1], ftop = 0.f, fsfc = 0.f, jsfc = 0.f;
+    for (int imu = 0; imu < nmus; ++imu) {
+        const float two_pi_w = 2.f * pi_value<float>() * float(kGaussWts[nmus - 1][imu]);
+        float tr[CL], sdn[CL], sup[CL];
+#pragma unroll
+        for (int i = 0; i < CL; ++i) { tr[i] = vt[i]; sdn[i] = vd[i]; sup[i] = vu[i]; }
+        // (a warp rewrites only its own slots, which only it has read since the scan)
+        lw_chunk_maps<float, CL>(tr, vl, sdn, sup, sm_a, sm_bd, sm_bu, w, lane, float(kGaussDs[nmus - 1][imu]));
+        __syncthreads();
+        if (w == 0) lw_chunk_scan<float>(a, sm_a, sm_bd, sm_bu, nw, lane, ic, g, two_pi_w);
+        __syncthreads();
+        float radn = sm_bd[w * 32 + lane], rup = sm_bu[w * 32 + lane], rjac = sm_a[w * 32 + lane];
+        auto add = [&](float& f, float r) { f = imu == 0 ? two_pi_w * r : f + two_pi_w * r; };
+        add(ftop, radn);
+        add(fsfc, rup);
+        if (JAC) add(jsfc, rjac);
+#pragma unroll
+        for (int i = 0; i < CL; ++i) {
+            radn = tr[i] * radn + sdn[i];
+            add(fdn[i], radn);
+        }
+#pragma unroll
+        for (int i = CL - 1; i >= 0; --i) {
+            rup = tr[i] * rup + sup[i];
+            add(fup[i], rup);
+            if (JAC) {
+                rjac *= tr[i];
+                add(fj[i], rjac);
+            }
+        }
+    }
+    if (!cv) return;
+    const size_t c0 = ic + size_t(g) * ncv;
+    auto lev = [&](int j) { return c0 + size_t(a.top_at_1 ? j : nlay - j) * ncol; };   // level j from the top
+    if (w == 0) a.flux_dn[lev(0)] = ftop;
+    if (w == nw - 1) {
+        a.flux_up[lev(nlay)] = fsfc;
+        if (JAC) a.flux_up_jac[lev(nlay)] = jsfc;
+    }
+#pragma unroll
+    for (int i = 0; i < CL; ++i)
+        if (j0 + i < nlay) {
+            a.flux_dn[lev(j0 + i + 1)] = fdn[i];
+            a.flux_up[lev(j0 + i)] = fup[i];
+            if (JAC) a.flux_up_jac[lev(j0 + i)] = fj[i];
+        }
 }
 
 // TMA-staged FP32 variant (nlay <= kLwTmaMaxLay).  A tile is the (32 columns x nlay layers)
@@ -801,9 +887,18 @@ int rte_lw(rrtmgp_b200_bands b, int ncol, int nlay, int top_at_1, const T* tau, 
     RB_CHECK_ARG(nmus >= 1 && nmus <= 4, "rte_lw: n_gauss_angles must be 1..4");
     RB_CHECK_ARG(tau && lay_src && lev_inc && lev_dec && sfc_src && sfc_emis && flux_up && flux_dn,
                  "rte_lw: null array");
+    const LwChunkArgs<T> a{ncol, nlay, b->nband, top_at_1, b->d_gpt2band, sfc_src, sfc_emis, inc_flux,
+                           sfc_src_jac, flux_up, flux_dn, flux_up_jac};
+    if constexpr (sizeof(T) == 4) {
+        if (nmus > 1 && nlay <= 8 * 16) {
+            const dim3 grid(ceil_div(ncol, 32), b->ngpt);
+            const auto kernel = flux_up_jac ? lw_solver_angles<true> : lw_solver_angles<false>;
+            kernel<<<grid, 32 * ceil_div(nlay, 8), 0, as_stream(stream)>>>(a, nmus, tau, lay_src, lev_inc, lev_dec);
+            RB_LAUNCH("lw_solver_angles");
+            return RRTMGP_B200_OK;
+        }
+    }
     if (nmus == 1 && nlay <= 16 * 16) {
-        const LwChunkArgs<T> a{ncol, nlay, b->nband, top_at_1, b->d_gpt2band, sfc_src, sfc_emis, inc_flux,
-                               sfc_src_jac, flux_up, flux_dn, flux_up_jac};
         const T* lev_dn = top_at_1 ? lev_inc : lev_dec;
         const T* lev_up = top_at_1 ? lev_dec : lev_inc;
         if constexpr (sizeof(T) == 4) {

@@ -265,6 +265,31 @@ def test_rte_lw(api, oracle_mod, tables, gpu, prec, top_at_1, nmu, with_inc):
     cmp_flux("flux_dn", N(gd), dn, prec)
 
 
+@pytest.mark.parametrize("top_at_1", [True, False])
+@pytest.mark.parametrize("ncol,nlay,nmu", [(33, 7, 2), (5, 9, 4), (40, 128, 3), (3, 129, 2)])
+def test_rte_lw_angles_fp32(api, oracle_mod, tables, gpu, top_at_1, ncol, nlay, nmu):
+    """Several angles in FP32: one partial chunk, a one-layer last chunk, the deepest columns of the
+    chunked kernel (16 chunks) and the first that run the per-(column, g-point) kernel; with an
+    incident flux and the Jacobian, at the FP32 flux tolerance of the other solver tests."""
+    import torch
+    dt = torch.float32
+    atm = S.make_atmosphere(ncol, nlay, seed=90 + nlay, clouds=False, top_at_1=top_at_1)
+    go = oracle_mod.GasOptics(tables["lw"], S.ATM_GASES).gas_optics_lw(
+        atm["play"], atm["plev"], atm["tlay"], atm["tsfc"], atm["gases"], atm["tlev"])
+    rng = np.random.default_rng(8)
+    emis, inc = rng.uniform(0.8, 1.0, (ncol, 16)), rng.uniform(0, 2, (256, ncol))
+    up, dn, jac = oracle_mod.rte_lw(tables["lw"]["bnd_limits_gpt"], go["tau"], top_at_1, go, emis, inc, nmu,
+                                    flux_up_jac=True)
+    kd = api.Gas_optics_rrtmgp(tables["lw"], S.ATM_GASES)
+    src = {k: T(v, dt, gpu) for k, v in go.items()}
+    args = (kd.bands, src["tau"], top_at_1, src, T(emis, dt, gpu), T(inc, dt, gpu), nmu)
+    gu, gd, gj = api.Rte_lw.rte_lw(*args, flux_up_jac=True)
+    g2 = api.Rte_lw.rte_lw(*args)
+    torch.cuda.synchronize()
+    for name, got, ref in (("up", gu, up), ("dn", gd, dn), ("jac", gj, jac), ("up", g2[0], up), ("dn", g2[1], dn)):
+        cmp_flux("flux_" + name, N(got), ref, "f32")
+
+
 def test_rte_lw_large_nlay_without_smem_stash(api, oracle_mod, tables, gpu):
     """nlay large enough that the up-sweep stash does not fit in shared memory in FP64."""
     import torch
@@ -289,7 +314,8 @@ def test_rte_lw_surface_temperature_jacobian(api, oracle_mod, tables, gpu, prec,
     """gpt_flux_up_jac (the reference's do_jacobians output) against the oracle's, and against
     the finite difference it stands for: gpt_flux_up at Tsfc + 1 K minus at Tsfc (the fluxes
     depend on Tsfc only through the surface source, linearly).  One angle runs the chunked
-    kernel up to 256 layers; three angles and 300 layers the per-(column, g-point) kernel."""
+    kernel up to 256 layers, three FP32 angles the one that keeps its inputs over the angles;
+    three FP64 angles and 300 layers run the per-(column, g-point) kernel."""
     import torch
     dt = dtypes()[prec]
     atm = S.make_atmosphere(NCOL, nlay, seed=23, clouds=False, top_at_1=top_at_1)
