@@ -43,8 +43,11 @@ class _LongwaveFn(torch.autograd.Function):
         gases["h2o"], gases["o3"] = h2o, o3
         atm["gases"] = gases
         clouds = lwp is not None
-        out = fused.solve_lw(atm, with_clouds=clouds)
-        res = tuple(out[k].clone() for k in ("flux_up", "flux_dn", "flux_net", "heating_rate"))
+        # outputs of its own, not copies of the solver's; no zeros for outputs without a gradient
+        nlay, ncol = static["play"].shape
+        out = fused.solve_lw(atm, with_clouds=clouds, out=fused.new_outputs("lw", static["play"], ncol, nlay))
+        res = tuple(out[k] for k in ("flux_up", "flux_dn", "flux_net", "heating_rate"))
+        ctx.set_materialize_grads(False)
         ctx.fused, ctx.atm, ctx.clouds = fused, atm, clouds
         ctx.save_for_backward(tlay, tlev, tsfc, h2o, o3)
         return res
@@ -192,8 +195,10 @@ class _ShortwaveFn(torch.autograd.Function):
         gases["h2o"], gases["o3"] = h2o, o3
         atm["gases"] = gases
         clouds = lwp is not None
-        out = fused.solve_sw(atm, with_clouds=clouds)
-        res = tuple(out[k].clone() for k in ("flux_up", "flux_dn", "flux_dn_dir", "flux_net", "heating_rate"))
+        nlay, ncol = static["play"].shape
+        out = fused.solve_sw(atm, with_clouds=clouds, out=fused.new_outputs("sw", static["play"], ncol, nlay))
+        res = tuple(out[k] for k in ("flux_up", "flux_dn", "flux_dn_dir", "flux_net", "heating_rate"))
+        ctx.set_materialize_grads(False)
         ctx.fused, ctx.atm, ctx.clouds = fused, atm, clouds
         ctx.save_for_backward(h2o, o3)
         return res

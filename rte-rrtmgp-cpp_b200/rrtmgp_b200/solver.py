@@ -183,18 +183,25 @@ class Fused_solver:
         key = (kind, ncol, nlay, like.device)
         o = self._out.get(key)
         if o is None:
-            o = {k: torch.empty((nlay + 1, ncol), dtype=torch.float32, device=like.device)
-                 for k in ("flux_up", "flux_dn", "flux_net", "flux_dn_dir")}
-            o["heating_rate"] = torch.empty((nlay, ncol), dtype=torch.float32, device=like.device)
+            o = self.new_outputs(kind, like, ncol, nlay)
             self._out[key] = o
         return o
 
-    def solve_lw(self, atm: dict, with_clouds: bool = True):
+    @staticmethod
+    def new_outputs(kind, like, ncol, nlay):
+        """Output tensors of one solve ("lw" or "sw")."""
+        names = ("flux_up", "flux_dn", "flux_net") + (("flux_dn_dir",) if kind == "sw" else ())
+        o = {k: torch.empty((nlay + 1, ncol), dtype=torch.float32, device=like.device) for k in names}
+        o["heating_rate"] = torch.empty((nlay, ncol), dtype=torch.float32, device=like.device)
+        return o
+
+    def solve_lw(self, atm: dict, with_clouds: bool = True, out: dict | None = None):
+        """out: tensors to write instead of the solver's own (new_outputs)."""
         from . import _abi
         play = atm["play"]
         assert play.dtype == torch.float32, "the fused path is FP32"
         nlay, ncol = play.shape
-        o = self._outputs("lw", play, ncol, nlay)
+        o = out if out is not None else self._outputs("lw", play, ncol, nlay)
         P = api._ptr
         arr, keep = api.Gas_optics_rrtmgp._gases(atm["gases"], ncol, nlay, atm["play"])
         c = self.base.clw if (with_clouds and self.base.clw is not None) else None
@@ -207,14 +214,15 @@ class Fused_solver:
         return {k: o[k] for k in ("flux_up", "flux_dn", "flux_net", "heating_rate")}
 
 
-    def solve_sw(self, atm: dict, with_clouds: bool = True, with_aerosols: bool = False):
+    def solve_sw(self, atm: dict, with_clouds: bool = True, with_aerosols: bool = False, out: dict | None = None):
         """with_aerosols: atm["aerosols"] {aermr01 .. aermr11} and atm["rh"] (nlay, ncol) through
-        the base solver's aerosol tables, inside the fused kernel (rrtmgp_b200_forward_sw_aer_f32)."""
+        the base solver's aerosol tables, inside the fused kernel (rrtmgp_b200_forward_sw_aer_f32).
+        out: as solve_lw."""
         from . import _abi
         play = atm["play"]
         assert play.dtype == torch.float32, "the fused path is FP32"
         nlay, ncol = play.shape
-        o = self._outputs("sw", play, ncol, nlay)
+        o = out if out is not None else self._outputs("sw", play, ncol, nlay)
         P = api._ptr
         arr, keep = api.Gas_optics_rrtmgp._gases(atm["gases"], ncol, nlay, atm["play"])
         c = self.base.csw if (with_clouds and self.base.csw is not None) else None
