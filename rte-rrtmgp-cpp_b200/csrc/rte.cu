@@ -906,9 +906,11 @@ int rte_lw(rrtmgp_b200_bands b, int ncol, int nlay, int top_at_1, const T* tau, 
                 return lw_solver_tma_launch(a, b->ngpt, tau, lay_src, lev_dn, lev_up, stream);
         }
         const dim3 grid(ceil_div(ncol, 32), b->ngpt);
-        // FP32 up to 128 layers: 8-layer chunks (more warps with fewer rows in flight each
-        // measured faster than 16 at 8192 x 128); FP64 and deeper columns: 16-layer chunks
-        if (sizeof(T) == 4 && nlay <= 8 * 16)
+        // 8-layer chunks in FP32 up to 128 layers (more warps with fewer rows in flight each measured
+        // faster than 16 at 8192 x 128) and in FP64 (88 registers, no spills; 16 layers spill) while two
+        // blocks share an SM: LW solve 1024 x 72 955 -> 913 us, 2000 x 40 1.01 -> 0.92 ms, but
+        // 1000 x 128 1.41 -> 1.46 ms
+        if (nlay <= (sizeof(T) == 4 ? 128 : 88))
             lw_solver_chunked<T, 8, 512><<<grid, 32 * ceil_div(nlay, 8), 0, as_stream(stream)>>>(
                 a, tau, lay_src, lev_inc, lev_dec);
         else
@@ -971,7 +973,13 @@ int rte_sw(rrtmgp_b200_bands b, int ncol, int nlay, int top_at_1, const T* tau, 
         const dim3 grid(ceil_div(ncol, 32), b->ngpt);
         const bool i32 = sw_index32(ncol, nlay, b->ngpt);
         if constexpr (fp64) {
-            sw_solver_chunked<T, 16, 256><<<grid, 32 * ceil_div(nlay, 16), 0, as_stream(stream)>>>(a, tau, ssa, g);
+            // 8-layer chunks: with 16 a column of 72 layers was 5 warps at 254 registers, alone on an SM
+            // (SW solve of 1024 x 72 1.43 ms); at 96 registers two blocks of up to 10 warps share it
+            // (0.98 ms; 1.19 at 128 registers).  Deeper columns have 11 - 16 warps at 128 (1000 x 128
+            // 1.87 -> 1.68 ms).
+            const int nw = ceil_div(nlay, 8);
+            const auto kernel = nw <= 10 ? sw_solver_chunked<T, 8, 320, 2> : sw_solver_chunked<T, 8, 512>;
+            kernel<<<grid, 32 * nw, 0, as_stream(stream)>>>(a, tau, ssa, g);
         } else if (nlay <= 128) {
             const auto kernel = i32 ? sw_solver_chunked<T, 8, 512, 2, true> : sw_solver_chunked<T, 8, 512, 2, false>;
             kernel<<<grid, 32 * ceil_div(nlay, 8), 0, as_stream(stream)>>>(a, tau, ssa, g);
