@@ -6,7 +6,8 @@
 // warps, each team computing one column with the fused per-column code of lw_column.cuh /
 // sw_column.cuh on its own slice of shared memory and its own hardware barrier (ids 1..P).
 // Tiles are numbered item by item, items in order of decreasing tile time, and the
-// persistent CTAs (one per SM at 128 registers x 512 threads) take the next tile from a
+// persistent CTAs (two per SM at 64 registers x 512 threads, one at 128 where their shared memory
+// does not fit twice) take the next tile from a
 // device counter, so long tiles go first and the short ones fill the tail.
 //
 // The reference has no batching of grids: its driver loops over column blocks of one grid
@@ -128,8 +129,12 @@ struct SwItemIo : ItemIo {
 };
 
 // DENSE: a k-distribution with more than three minor intervals over some g-point (tau_abs).
-template <bool DENSE>
-__global__ void __launch_bounds__(kBatchThreads, 1)
+// PER_SM: CTAs per SM.  The column code waits on table loads and barriers, so two CTAs of 16 warps at
+// 64 registers (with spills) beat one at 128 although the tiles are the same: 12.4 -> 11.9 ms for 7
+// grids of 64 - 3000 columns and 40 - 200 layers (one CTA of 24 warps at 80 registers, with wider
+// tiles, 10.5 ms; tile shapes are kept within 16 warps).
+template <bool DENSE, int PER_SM>
+__global__ void __launch_bounds__(kBatchThreads, PER_SM)
 batch_forward_kernel(const KdistView<float> klw, const KdistView<float> ksw, const BatchItem* __restrict__ items,
                      const long long* __restrict__ tile_start, const int* __restrict__ tile_item, int nitems,
                      unsigned long long* __restrict__ counter)
@@ -242,6 +247,7 @@ struct rrtmgp_b200_batch_t {
     int nsm = 0, device = 0;
     bool dense = false;                // a k-distribution needs the DENSE kernel
     int max_smem = 0;                  // dynamic shared memory per CTA the kernel may use
+    int static_smem = 0, sm_smem = 0;  // the kernel's own, and an SM's
     // planned state
     bool dirty = true;
     std::vector<BatchItem> order;      // planned items in work order
@@ -275,33 +281,43 @@ size_t team_smem_bytes(const rrtmgp_b200_batch_t* b, int domain, int nlay, int c
     return align16(L.total);
 }
 
-// Largest P for a shape, 0 when the chunk length cannot hold nlay.
-int max_columns(const rrtmgp_b200_batch_t* b, int domain, int nlay, int cl)
+// Largest P for a shape whose teams have smem bytes together, 0 when the chunk length cannot hold
+// nlay or no team fits.
+int columns_in(const rrtmgp_b200_batch_t* b, int domain, int nlay, int cl, int smem)
 {
     const int W = ceil_div_i(nlay, cl);
     if (W > kBatchWarps) return 0;
     const size_t per = team_smem_bytes(b, domain, nlay, cl);
-    return int(std::min<size_t>(std::min(kBatchWarps / W, kMaxTeams), size_t(b->max_smem) / per));
+    return int(std::min<size_t>(std::min(kBatchWarps / W, kMaxTeams), size_t(std::max(smem, 0)) / per));
+}
+
+int max_columns(const rrtmgp_b200_batch_t* b, int domain, int nlay, int cl)
+{
+    return columns_in(b, domain, nlay, cl, b->max_smem);
 }
 
 // Shape of (domain, bin) for a grid of nlay layers: the stored shape when it fits, else the
-// heuristic (most busy warps, then the shorter chunk).
+// heuristic (most busy warps, then the shorter chunk; among the shapes that let two CTAs share an
+// SM, if there is one).
 TileShape shape_for(const rrtmgp_b200_batch_t* b, int domain, int nlay)
 {
     const int bin = ceil_div_i(nlay, 8);
     TileShape s = b->shape[domain][bin];
     if (s.cl && s.P >= 1 && s.P <= max_columns(b, domain, nlay, s.cl)) return s;
     TileShape best;
-    int best_busy = -1;
-    for (int cl : {8, 16}) {
-        const int P = max_columns(b, domain, nlay, cl);
-        if (P < 1) continue;
-        const int busy = P * ceil_div_i(nlay, cl);
-        if (busy > best_busy) {
-            best_busy = busy;
-            best.cl = cl;
-            best.P = P;
+    for (const int smem : {b->sm_smem / 2 - b->static_smem - 1024, b->max_smem}) {
+        int best_busy = -1;
+        for (int cl : {8, 16}) {
+            const int P = columns_in(b, domain, nlay, cl, smem);
+            if (P < 1) continue;
+            const int busy = P * ceil_div_i(nlay, cl);
+            if (busy > best_busy) {
+                best_busy = busy;
+                best.cl = cl;
+                best.P = P;
+            }
         }
+        if (best.cl) break;
     }
     return best;
 }
@@ -322,6 +338,17 @@ BatchItem planned(const rrtmgp_b200_batch_t* b, const BatchItem& in, const TileS
     it.W = ceil_div_i(it.nlay, s.cl);
     it.team_smem = int(team_smem_bytes(b, it.domain, it.nlay, s.cl));
     return it;
+}
+
+// CTAs per SM (the PER_SM instance) of a launch with smem bytes per CTA.
+int per_sm(const rrtmgp_b200_batch_t* b, size_t smem)
+{
+    return 2 * (smem + size_t(b->static_smem) + 1024) <= size_t(b->sm_smem) ? 2 : 1;
+}
+
+int persistent_ctas(const rrtmgp_b200_batch_t* b, size_t smem, long long ntiles)
+{
+    return int(std::min<long long>((long long)b->nsm * per_sm(b, smem), std::max<long long>(ntiles, 1)));
 }
 
 void release_graph(rrtmgp_b200_batch_t* b)
@@ -403,7 +430,7 @@ int plan(rrtmgp_b200_batch_t* b)
     for (auto& kv : keyed) b->order.push_back(kv.second);
     int st = upload(b, b->order, b->ntiles, b->smem);
     if (st) return st;
-    b->ctas = int(std::min<long long>(b->nsm, std::max<long long>(b->ntiles, 1)));
+    b->ctas = persistent_ctas(b, b->smem, b->ntiles);
     b->dirty = false;
     return RRTMGP_B200_OK;
 }
@@ -412,15 +439,13 @@ int launch_persistent(rrtmgp_b200_batch_t* b, const BatchItem* d_items, const lo
                       long long ntiles, size_t smem, cudaStream_t s)
 {
     RB_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), s), "batch: counter reset");
-    const int ctas = int(std::min<long long>(b->nsm, std::max<long long>(ntiles, 1)));
+    const int ctas = persistent_ctas(b, smem, ntiles);
     const KdistView<float> klw = b->k[0] ? b->k[0]->v32 : KdistView<float>{};
     const KdistView<float> ksw = b->k[1] ? b->k[1]->v32 : KdistView<float>{};
-    if (b->dense)
-        batch_forward_kernel<true><<<ctas, kBatchThreads, smem, s>>>(klw, ksw, d_items, d_starts, b->d_tile_item, nitems,
-                                                                     b->d_counter);
-    else
-        batch_forward_kernel<false><<<ctas, kBatchThreads, smem, s>>>(klw, ksw, d_items, d_starts, b->d_tile_item,
-                                                                      nitems, b->d_counter);
+    const bool two = per_sm(b, smem) == 2;
+    const auto kernel = b->dense ? (two ? batch_forward_kernel<true, 2> : batch_forward_kernel<true, 1>)
+                                 : (two ? batch_forward_kernel<false, 2> : batch_forward_kernel<false, 1>);
+    kernel<<<ctas, kBatchThreads, smem, s>>>(klw, ksw, d_items, d_starts, b->d_tile_item, nitems, b->d_counter);
     RB_LAUNCH("batch_forward_kernel");
     return RRTMGP_B200_OK;
 }
@@ -541,12 +566,16 @@ int batch_create(rrtmgp_b200_kdist klw, rrtmgp_b200_cloud clw, rrtmgp_b200_kdist
     int optin = 0;
     RB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device), "batch_create");
     b->dense = (klw && klw->v32.max_minor_per_g > 3) || (ksw && ksw->v32.max_minor_per_g > 3);
-    const auto kernel = b->dense ? batch_forward_kernel<true> : batch_forward_kernel<false>;
-    cudaFuncAttributes fa{};
-    RB_CUDA(cudaFuncGetAttributes(&fa, kernel), "batch_create");
-    b->max_smem = optin - int(fa.sharedSizeBytes);
-    RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b->max_smem),
-            "batch_create: kernel attribute");
+    RB_CUDA(cudaDeviceGetAttribute(&b->sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->device), "batch_create");
+    for (const auto kernel : {b->dense ? batch_forward_kernel<true, 1> : batch_forward_kernel<false, 1>,
+                              b->dense ? batch_forward_kernel<true, 2> : batch_forward_kernel<false, 2>}) {
+        cudaFuncAttributes fa{};
+        RB_CUDA(cudaFuncGetAttributes(&fa, kernel), "batch_create");
+        b->static_smem = int(fa.sharedSizeBytes);
+        b->max_smem = optin - b->static_smem;
+        RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b->max_smem),
+                "batch_create: kernel attribute");
+    }
     for (const BatchItem& it : b->items)
         if (!shape_for(b.get(), it.domain, it.nlay).cl)
             return fail(RRTMGP_B200_ERR_UNSUPPORTED, "batch_create: shared memory need too large for nlay = " +
@@ -612,7 +641,7 @@ int batch_autotune(rrtmgp_b200_batch_t* b, int reps, cudaStream_t s)
                     if (st) break;
                     const float col_us = 1000.f * ms_min / float(copies * it.ncol);
                     if (!best.cl || col_us < best_col_us) {
-                        const int ctas = int(std::min<long long>(b->nsm, ntiles));
+                        const int ctas = persistent_ctas(b, smem, ntiles);
                         best = cand;
                         best.tile_us = 1000.f * ms_min * float(ctas) / float(ntiles);
                         best_col_us = col_us;
