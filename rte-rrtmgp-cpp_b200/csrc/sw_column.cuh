@@ -15,11 +15,12 @@
 //   2. barrier; every warp forms its direct flux at the chunk top from the PT of the chunks
 //      above, emits the direct fluxes and direct absorption of its layers and scales its
 //      composite's sources to absolute values;
-//   3. barrier; every warp walks the composites from the surface up: albedo and upward
-//      source at its chunk bottom, and the affine maps fd_bot = F fd_top + G of the chunks
-//      above it, composed into its incident diffuse flux;
-//   4. pass 2 (bottom-up within the chunk): albedo and source per level (adding_kernel);
-//      pass 3 (top-down): diffuse down/up fluxes per level and per-layer diffuse absorption;
+//   3. barrier; two warps scan the composites of all chunks, from the surface up and from the
+//      top down; barrier; every warp takes the albedo and upward source below its chunk and
+//      closes the two sides at its top into its incident diffuse flux;
+//   4. pass 2 (bottom-up within the chunk): albedo and source per level (adding_kernel) and each
+//      layer's transfer of the downward flux; pass 3 (top-down): diffuse down/up fluxes per
+//      level and per-layer diffuse absorption;
 //   5. warp reduce-scatter over the 32 g-points, FP64 accumulation per lane.
 // Heating rates use the per-layer absorbed flux (direct: F_dir (1 - Tn - Rdir - Tdir);
 // diffuse: (F_dn(top) + F_up(bottom)) (1 - R - T)), which equals the net-flux divergence of
@@ -233,9 +234,9 @@ __device__ __forceinline__ void sw_forward_column(const Cx& cx, const KdistView<
         //    (sm_above: no diffuse flux at the top of the atmosphere).  At an interface the two
         //    sides close: f_dn = (D + Rd src) / (1 - Rd alb).  Both scans are chains of NW
         //    divisions on which the whole CTA waits, so they run side by side and load a chunk ahead
-        //    (one warp doing the upward scan and then walking the fluxes back down: 8192 x 128
-        //    SW forward 4.05 -> 3.86 ms, with the layer transfers below kept from pass 2); with every warp scanning all chunks itself they were
-        //    O(chunks^2) instructions per group.
+        //    (8192 x 128 SW forward 4.05 -> 3.86 ms against one warp doing the upward scan and then
+        //    walking the fluxes back down, the layer transfers of pass 2 included); with every warp
+        //    scanning all chunks itself they were O(chunks^2) instructions per group.
         const float ad = gv ? __ldg(io.alb_dir() + gband + size_t(cx.icol()) * nband) : 0.f;
         const float af = gv ? __ldg(io.alb_dif() + gband + size_t(cx.icol()) * nband) : 0.f;
         if (w == 0) {
