@@ -91,7 +91,7 @@ __device__ __forceinline__ Dual<N> operator-(const Dual<N>& a)
 {
     return 0.f - a;
 }
-// Quotient; fast = the __fdividef value (as the fused forward), else IEEE division.
+// Quotient; fast = the fast_div value (as the fused forward), else IEEE division.
 template <int N>
 __device__ __forceinline__ Dual<N> ddiv(const Dual<N>& a, const Dual<N>& b, bool fast)
 {
