@@ -190,18 +190,33 @@ class Fused_solver:
     @staticmethod
     def new_outputs(kind, like, ncol, nlay):
         """Output tensors of one solve ("lw" or "sw")."""
+        return {k: torch.empty(shape, dtype=torch.float32, device=like.device)
+                for k, shape in Fused_solver._output_shapes(kind, ncol, nlay)}
+
+    @staticmethod
+    def _output_shapes(kind, ncol, nlay):
         names = ("flux_up", "flux_dn", "flux_net") + (("flux_dn_dir",) if kind == "sw" else ())
-        o = {k: torch.empty((nlay + 1, ncol), dtype=torch.float32, device=like.device) for k in names}
-        o["heating_rate"] = torch.empty((nlay, ncol), dtype=torch.float32, device=like.device)
-        return o
+        return [(k, (nlay + 1, ncol)) for k in names] + [("heating_rate", (nlay, ncol))]
+
+    @staticmethod
+    def _check_outputs(kind, out, like, ncol, nlay):
+        """out, if it holds every output as the kernels write it; they see only addresses, so a short
+        or FP64 tensor would be written past its end."""
+        for k, shape in Fused_solver._output_shapes(kind, ncol, nlay):
+            t = out.get(k)
+            if (t is None or t.shape != shape or t.dtype != torch.float32 or t.device != like.device
+                    or not t.is_contiguous()):
+                raise ValueError(f"out[{k!r}]: a contiguous float32 tensor of shape {shape} on {like.device} is needed")
+        return out
 
     def solve_lw(self, atm: dict, with_clouds: bool = True, out: dict | None = None):
-        """out: tensors to write instead of the solver's own (new_outputs)."""
+        """out: tensors to write instead of the solver's own (new_outputs); others raise ValueError."""
         from . import _abi
         play = atm["play"]
         assert play.dtype == torch.float32, "the fused path is FP32"
         nlay, ncol = play.shape
-        o = out if out is not None else self._outputs("lw", play, ncol, nlay)
+        o = (self._outputs("lw", play, ncol, nlay) if out is None
+             else self._check_outputs("lw", out, play, ncol, nlay))
         P = api._ptr
         arr, keep = api.Gas_optics_rrtmgp._gases(atm["gases"], ncol, nlay, atm["play"])
         c = self.base.clw if (with_clouds and self.base.clw is not None) else None
@@ -222,7 +237,8 @@ class Fused_solver:
         play = atm["play"]
         assert play.dtype == torch.float32, "the fused path is FP32"
         nlay, ncol = play.shape
-        o = out if out is not None else self._outputs("sw", play, ncol, nlay)
+        o = (self._outputs("sw", play, ncol, nlay) if out is None
+             else self._check_outputs("sw", out, play, ncol, nlay))
         P = api._ptr
         arr, keep = api.Gas_optics_rrtmgp._gases(atm["gases"], ncol, nlay, atm["play"])
         c = self.base.csw if (with_clouds and self.base.csw is not None) else None

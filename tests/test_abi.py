@@ -135,3 +135,28 @@ def test_gas_concentrations_are_validated_before_any_pointer_is_taken():
         api.Gas_optics_rrtmgp._gases({"o3": torch.ones((ncol, nlay), dtype=torch.float32)}, ncol, nlay, play)
     with pytest.raises(ValueError, match="torch tensor"):
         api.Gas_optics_rrtmgp._gases({"co2": np.ones(1, np.float32)}, ncol, nlay, play)
+
+
+@pytest.mark.parametrize("kind", ["lw", "sw"])
+@pytest.mark.parametrize("fault", ["short", "flat", "double", "strided", "device", "missing"])
+def test_fused_solver_refuses_outputs_it_cannot_write(kind, fault):
+    """solve_lw / solve_sw hand the addresses of out= to the kernels: tensors of another size, type,
+    device or stride, or a missing one, are refused before the library is called (no solver and
+    no GPU behind this call)."""
+    import torch
+    from rrtmgp_b200.solver import Fused_solver
+    nlay, ncol = 6, 4
+    atm = {"play": torch.ones(nlay, ncol)}
+    solve = getattr(Fused_solver(None), "solve_" + kind)
+    for name in Fused_solver.new_outputs(kind, atm["play"], ncol, nlay):
+        out = Fused_solver.new_outputs(kind, atm["play"], ncol, nlay)
+        n = out[name].shape[0]
+        bad = {"short": torch.empty(n - 1, ncol), "flat": torch.empty(n * ncol), "double": out[name].double(),
+               "strided": torch.empty(ncol, n).T, "device": torch.empty(n, ncol, device="meta"), "missing": None}[fault]
+        out[name] = bad
+        if bad is None:
+            del out[name]
+        with pytest.raises(ValueError, match=f"out\\['{name}'\\]"):
+            solve(atm, out=out)
+    good = Fused_solver.new_outputs(kind, atm["play"], ncol, nlay)
+    assert Fused_solver._check_outputs(kind, good, atm["play"], ncol, nlay) is good
