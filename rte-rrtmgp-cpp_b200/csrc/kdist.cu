@@ -304,31 +304,36 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
                             make_float2(float(m.kminor[(size_t(it) * ne + ie) * nc + c]),
                                         float(m.kminor[(size_t(it) * ne + ie + 1) * nc + c]));
         }
-        // Intervals covering each g-point, as codes (contributor << kScalBits) | scaling kind,
-        // in the file order of the intervals.
-        std::vector<std::vector<int>> codes[2];
+        // Intervals covering each g-point in their file order.  Contributor and scaling kind stay apart on
+        // the host: with more than kMaxScal kinds (which the packed kernels refuse) the kind
+        // does not fit the bits that a code has for it.
+        struct Cover {
+            int c, kind;
+            int code() const { return (c << kScalBits) | (kind & (kMaxScal - 1)); }
+        };
+        std::vector<std::vector<Cover>> cover[2];
         for (int atm = 0; atm < 2; ++atm) {
             const MinorHost& m = mh[atm];
-            codes[atm].assign(ng, {});
+            cover[atm].assign(ng, {});
             for (size_t im = 0; im < m.gstart.size(); ++im)
                 for (int g = m.gstart[im]; g < m.gend[im]; ++g)
-                    codes[atm][g].push_back(((m.kstart[im] + g - m.gstart[im]) << kScalBits) | sid[atm][im]);
-            for (int g = 0; g < ng; ++g) v.max_minor_per_g = std::max(v.max_minor_per_g, int(codes[atm][g].size()));
+                    cover[atm][g].push_back({m.kstart[im] + g - m.gstart[im], sid[atm][im]});
+            for (int g = 0; g < ng; ++g) v.max_minor_per_g = std::max(v.max_minor_per_g, int(cover[atm][g].size()));
         }
         v.minor_gx_stride = std::max(v.max_minor_per_g - 3, 0);
         for (int atm = 0; atm < 2; ++atm) {
             mg[atm].assign(ng, make_int4(0, 0, 0, 0));
             if (v.minor_gx_stride) mgx[atm].assign(size_t(ng) * v.minor_gx_stride, 0);
             for (int g = 0; g < ng; ++g) {
-                const std::vector<int>& c = codes[atm][g];
+                const std::vector<Cover>& c = cover[atm][g];
                 int4& e = mg[atm][g];
                 e.x = int(c.size());
                 // unused slots repeat the first one, so a kernel may read every slot below a
                 // warp-wide maximum count and discard the extra terms
-                e.y = c.empty() ? 0 : c[0];
-                e.z = c.size() > 1 ? c[1] : e.y;
-                e.w = c.size() > 2 ? c[2] : e.y;
-                for (size_t n = 3; n < c.size(); ++n) mgx[atm][size_t(g) * v.minor_gx_stride + n - 3] = c[n];
+                e.y = c.empty() ? 0 : c[0].code();
+                e.z = c.size() > 1 ? c[1].code() : e.y;
+                e.w = c.size() > 2 ? c[2].code() : e.y;
+                for (size_t n = 3; n < c.size(); ++n) mgx[atm][size_t(g) * v.minor_gx_stride + n - 3] = c[n].code();
             }
         }
         if (info.has_rayleigh) {
@@ -355,11 +360,11 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
             const double* rayl = !info.has_rayleigh ? nullptr : (atm == 0 ? t->rayl_lower : t->rayl_upper);
             for (int u = 0; u < nu; ++u)
                 for (int g = 0; g < ng; ++g) {
-                    const std::vector<int>& c = codes[atm][g];
+                    const std::vector<Cover>& c = cover[atm][g];
                     int sids = 0;
                     for (int q = 0; q < 2; ++q) {
                         const int n = 2 * u + q - r0;   // interval of this pair, -1: Rayleigh
-                        if (n >= 0 && n < int(c.size())) sids |= (c[n] & (kMaxScal - 1)) << (8 * q);
+                        if (n >= 0 && n < int(c.size())) sids |= (c[n].kind & (kMaxScal - 1)) << (8 * q);
                         if (n >= int(c.size()) || (n < 0 && !rayl)) continue;
                         for (int it = 0; it < nt; ++it)
                             for (int ie = 0; ie < ne - 1; ++ie) {
@@ -367,7 +372,7 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
                                 for (int e = 0; e < 2; ++e) {
                                     const size_t row = size_t(it) * ne + ie + e;
                                     const float v1 = n < 0 ? float(rayl[row * ng + g])
-                                                           : float(m.kminor[row * nc + (c[n] >> kScalBits)]);
+                                                           : float(m.kminor[row * nc + c[n].c]);
                                     (q == 0 ? (e == 0 ? o.x : o.y) : (e == 0 ? o.z : o.w)) = v1;
                                 }
                             }

@@ -160,3 +160,26 @@ def test_fused_solver_refuses_outputs_it_cannot_write(kind, fault):
             solve(atm, out=out)
     good = Fused_solver.new_outputs(kind, atm["play"], ncol, nlay)
     assert Fused_solver._check_outputs(kind, good, atm["play"], ncol, nlay) is good
+
+
+def test_kdist_with_many_scaling_kinds_stays_in_its_tables(tmp_path):
+    """More scaling kinds than a minor-interval code has bits for (the packed kernels refuse such a
+    layout, the general ones take it): laying the tables out on the host reads inside them.  The
+    address sanitizer sees a read past the end; run without a device, whether there is one or
+    not."""
+    import os
+    import shutil
+    import subprocess
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not Path(nvcc).exists():
+        pytest.skip("needs nvcc")
+    root = HEADER.parent.parent
+    csrc = root / "rte-rrtmgp-cpp_b200" / "csrc"
+    exe = tmp_path / "driver"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O1", "-std=c++17", "--expt-relaxed-constexpr",
+                    "-Xcompiler", "-fsanitize=address", "-I", str(HEADER.parent), "-I", str(csrc), "-o", str(exe),
+                    str(root / "tests" / "cpp" / "kdist_kinds_driver.cpp"), str(csrc / "kdist.cu")],
+                   check=True, capture_output=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True,
+                       env={**os.environ, "CUDA_VISIBLE_DEVICES": "", "ASAN_OPTIONS": "protect_shadow_gap=0:detect_leaks=0"})
+    assert r.returncode == 0, r.stdout + r.stderr[:2000]
