@@ -401,8 +401,7 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
         pack_corners_kernel<<<ceil_div(long(nrow), 256), 256>>>(
             t->ntemp, t->npres, t->neta, t->ngpt, v.kmajor, t->planck_frac ? v.planck_frac : nullptr,
             const_cast<float4*>(v.kmaj4), const_cast<float4*>(v.pfrac4), const_cast<Tab8*>(v.kmp8));
-        RB_LAUNCH("pack_corners_kernel");
-        RB_CUDA(cudaStreamSynchronize(nullptr), "pack_corners_kernel");   // the handle may be used on any stream
+        RB_LAUNCH("pack_corners_kernel");   // kdist_create waits for it
     }
     return RRTMGP_B200_OK;
 }
@@ -646,6 +645,13 @@ int rrtmgp_b200_kdist_create(const rrtmgp_b200_kdist_tables* t, const char* cons
     }
     k->v32.solar_source = k->d_solar32;
     k->v64.solar_source = k->d_solar64;
+    // Copies from pageable memory, memsets and the packing kernel may still be under way on the legacy
+    // stream, which non-blocking streams do not wait for; the handle may be used on any stream.
+    const cudaError_t done = cudaStreamSynchronize(nullptr);
+    if (done != cudaSuccess) {
+        *out = nullptr;
+        return bail(cuda_status(done, "kdist_create"));
+    }
     *out = k;
     return RRTMGP_B200_OK;
 }

@@ -142,6 +142,38 @@ def test_gas_optics_lw_band_crossing_minor(api, oracle_mod, tables, gpu, prec):
         assert e.value.status == ERR_UNSUPPORTED
 
 
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("kind", ["lw", "sw"])
+def test_new_handle_on_a_non_blocking_stream(api, tables, gpu, prec, kind):
+    """The first call on a new handle, on a stream that does not wait for the legacy one (torch's own):
+    creation has waited for its uploads and its packing kernel, so the outputs equal those of
+    the same call after a device synchronisation, bit for bit, in both precisions (the FP64
+    tables are uploaded last)."""
+    import torch
+    dt = dtypes()[prec]
+    atm = S.make_atmosphere(NCOL, NLAY, seed=19, clouds=False)
+    a = {k: T(atm[k], dt, gpu) for k in ("play", "plev", "tlay", "tlev", "tsfc")}
+    g = gas_dict(atm, dt, gpu)
+
+    def call(kd):
+        if kind == "lw":
+            o = kd.gas_optics_lw(a["play"], a["plev"], a["tlay"], a["tsfc"], g, a["tlev"], None)
+        else:
+            o = kd.gas_optics_sw(a["play"], a["plev"], a["tlay"], g, None)
+        return {k: v for k, v in o.items() if torch.is_tensor(v)}
+
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream(device=gpu)
+    with torch.cuda.stream(s):
+        kd = api.Gas_optics_rrtmgp(tables[kind], S.ATM_GASES)
+        first = call(kd)
+    torch.cuda.synchronize()
+    again = call(kd)
+    torch.cuda.synchronize()
+    for k in again:
+        assert torch.equal(first[k], again[k]), k
+
+
 def test_gas_profile_and_scalar_inputs(api, oracle_mod, tables, gpu):
     """Gas_concs accepts scalars, (1, nlay) profiles and (ncol, nlay) fields."""
     import torch
