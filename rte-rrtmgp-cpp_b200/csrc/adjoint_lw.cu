@@ -630,8 +630,9 @@ lw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const AdjClo
     if (CLUSTER) cluster.sync();   // no CTA leaves while its shared memory may still be read remotely
 }
 
-// Up to 128 layers (CL = 8) or 256 (CL = 16, if the records fit) one CTA of ceil(nlay / CL)
-// warps per column; beyond, clusters of CS = ceil(nlay / 128) CTAs of 16 warps (CL = 8).
+// Up to 128 layers one CTA of ceil(nlay / CL) warps per column, with two buffers of chunk maps;
+// beyond, clusters of CS = ceil(nlay / 128) CTAs of 16 warps (CL = 8) with one.  The buffer count goes
+// with the kernel (CLUSTER), so a one-CTA column whose two buffers do not fit is refused.
 template <int CL, bool FLUX, bool DENSE>
 int launch_lw_adjoint(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay, int idx_o3, const float* play,
                       const float* plev, const float* tlay, const float* tlev, const float* tsfc, const float* col_dry,
@@ -645,7 +646,7 @@ int launch_lw_adjoint(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     RB_CHECK_ARG(CL == 8 || NW1 <= 8, "adjoint_lw: chunk 16 covers at most 128 layers");
     int CS = 1, NWc = NW1;
     size_t smem = smem1;
-    if (NW1 > 16 || smem1 > 227 * 1024) {
+    if (NW1 > 16) {
         RB_CHECK_ARG(CL == 8, "adjoint_lw: columns deeper than one CTA holds need chunk 8");
         NWc = 16;
         CS = (nlay + 16 * CL - 1) / (16 * CL);

@@ -14,6 +14,7 @@ import pytest
 from rrtmgp_b200 import synthetic as S
 
 from test_gpu_adjoint import _check, _fd, _fd_bands, _get, _informative, _seeds, _sw_seeds
+from test_gpu_scale import _take
 from test_gpu_stages import N, T, cmp, dtypes
 
 pytestmark = pytest.mark.gpu
@@ -110,6 +111,38 @@ def test_lw_adjoint_dense_matches_fd(oracle_mod, dense, gpu):
     got = {k: v.double().cpu().numpy() for k, v in g.items()}
     for key in ("tlay", "tlev", "tsfc", "h2o", "o3"):
         _check(f"dense lw d/d{key}", got[key], _fd(fwd, atm, seeds, key), _informative(_get(atm, key)))
+
+
+def test_lw_adjoint_dense_shared_memory_limit(oracle_mod, dense, gpu):
+    """The dense tables' longwave adjoint at the shared-memory limit of one CTA per column: 120 layers
+    (15 chunks, 228400 of 232448 bytes) run, for few columns, whose g-points are split, and for
+    many, and match central differences; 121 and 128 layers need 243600 bytes and are refused
+    before any launch."""
+    import torch
+    from rrtmgp_b200._abi import ERR_UNSUPPORTED, RrtmgpError
+    from rrtmgp_b200.autodiff import adjoint_lw
+    from rrtmgp_b200.solver import atm_to_device
+    rng = np.random.default_rng(21)
+    base, fused = _solvers(dense)
+    for nlay in (121, 128):
+        for ncol in (3, 400):
+            big = atm_to_device(S.make_atmosphere(ncol, nlay, seed=3, clouds=True, trace_gases=True), torch.float32, gpu)
+            up = torch.ones((nlay + 1, ncol), device=gpu)
+            for with_fluxes in (False, True):
+                with pytest.raises(RrtmgpError) as e:
+                    adjoint_lw(fused, big, up, up, None, with_fluxes=with_fluxes)
+                assert e.value.status == ERR_UNSUPPORTED
+    ncol, nlay = 400, 120
+    atm, seeds, cols = S.make_atmosphere(ncol, nlay, seed=22, clouds=True, trace_gases=True), _seeds(nlay, ncol, rng), [0, 399]
+    few, few_seeds = _take(atm, cols), {k: np.ascontiguousarray(v[:, cols]) for k, v in seeds.items()}
+    kd, cl = oracle_mod.GasOptics(dense["lw"], GASES), oracle_mod.CloudOptics(dense["cloud_lw"])
+    ref = {k: _fd(lambda a: oracle_mod.forward_lw(kd, cl, a), few, few_seeds, k) for k in ("tlay", "tsfc")}
+    for a, s, pick in ((few, few_seeds, [0, 1]), (atm, seeds, cols)):
+        t = {k: torch.as_tensor(v, dtype=torch.float32, device=gpu).contiguous() for k, v in s.items()}
+        g = adjoint_lw(fused, atm_to_device(a, torch.float32, gpu), t["flux_up"], t["flux_dn"], t["heating_rate"])
+        for k in ref:
+            got = g[k].double().cpu().numpy()[..., pick]
+            _check(f"dense lw {a['ncol']} x 120 d/d{k}", got, ref[k], _informative(_get(few, k)))
 
 
 def test_sw_adjoint_dense_matches_fd(oracle_mod, dense, gpu):
