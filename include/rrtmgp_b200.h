@@ -647,6 +647,9 @@ int rrtmgp_b200_batch_run(rrtmgp_b200_batch b, int mode, void* stream);
  * timed runs each, the fastest counts) and keeps the fastest.  Synchronous.  Run it with the
  * inputs filled: the sample writes the outputs of the sampled grids. */
 int rrtmgp_b200_batch_autotune(rrtmgp_b200_batch b, int reps, void* stream);
+/* CTAs per SM (1 or 2) of the batch's launches as its grids and tables have it; the tuner times the
+ * shapes that fit this many.  A launch takes one where a stored shape does not fit twice. */
+int rrtmgp_b200_batch_ctas_per_sm(rrtmgp_b200_batch b, int* ctas);
 /* Tile shape of domain (0 longwave, 1 shortwave) for nlay in [8 bin - 7, 8 bin], bin 1..32:
  * chunk (8 or 16 layers per warp), columns per CTA, and the time of one tile in
  * microseconds (the work order key; 0 before any autotune).  set_plan validates the shape. */

@@ -6,8 +6,8 @@
 // warps, each team computing one column with the fused per-column code of lw_column.cuh /
 // sw_column.cuh on its own slice of shared memory and its own hardware barrier (ids 1..P).
 // Tiles are numbered item by item, items in order of decreasing tile time, and the
-// persistent CTAs (two per SM at 64 registers x 512 threads, one at 128 where their shared memory
-// does not fit twice) take the next tile from a
+// persistent CTAs (one per SM at 128 registers x 512 threads, two at 64 where one would leave
+// warps idle: ctas_per_sm) take the next tile from a
 // device counter, so long tiles go first and the short ones fill the tail.
 //
 // The reference has no batching of grids: its driver loops over column blocks of one grid
@@ -129,10 +129,7 @@ struct SwItemIo : ItemIo {
 };
 
 // DENSE: a k-distribution with more than three minor intervals over some g-point (tau_abs).
-// PER_SM: CTAs per SM.  The column code waits on table loads and barriers, so two CTAs of 16 warps at
-// 64 registers (with spills) beat one at 128 although the tiles are the same: 12.4 -> 11.9 ms for 7
-// grids of 64 - 3000 columns and 40 - 200 layers (one CTA of 24 warps at 80 registers, with wider
-// tiles, 10.5 ms; tile shapes are kept within 16 warps).
+// PER_SM: CTAs per SM, at 128 or at 64 registers (with spills): ctas_per_sm.
 template <bool DENSE, int PER_SM>
 __global__ void __launch_bounds__(kBatchThreads, PER_SM)
 batch_forward_kernel(const KdistView<float> klw, const KdistView<float> ksw, const BatchItem* __restrict__ items,
@@ -254,6 +251,7 @@ struct rrtmgp_b200_batch_t {
     std::vector<long long> starts;
     long long ntiles = 0;
     int ctas = 0;
+    int per_sm = 1;                    // CTAs per SM of the launch (the PER_SM instance)
     size_t smem = 0;
     BatchItem* d_items = nullptr;
     long long* d_starts = nullptr;
@@ -281,6 +279,12 @@ size_t team_smem_bytes(const rrtmgp_b200_batch_t* b, int domain, int nlay, int c
     return align16(L.total);
 }
 
+// Dynamic shared memory of a CTA in a launch with per_sm CTAs per SM (an SM keeps 1 KB per CTA).
+int smem_limit(const rrtmgp_b200_batch_t* b, int per_sm)
+{
+    return std::min(b->max_smem, b->sm_smem / per_sm - b->static_smem - 1024);
+}
+
 // Largest P for a shape whose teams have smem bytes together, 0 when the chunk length cannot hold
 // nlay or no team fits.
 int columns_in(const rrtmgp_b200_batch_t* b, int domain, int nlay, int cl, int smem)
@@ -296,30 +300,67 @@ int max_columns(const rrtmgp_b200_batch_t* b, int domain, int nlay, int cl)
     return columns_in(b, domain, nlay, cl, b->max_smem);
 }
 
-// Shape of (domain, bin) for a grid of nlay layers: the stored shape when it fits, else the
-// heuristic (most busy warps, then the shorter chunk; among the shapes that let two CTAs share an
-// SM, if there is one).
-TileShape shape_for(const rrtmgp_b200_batch_t* b, int domain, int nlay)
+// Heuristic shape for a grid of nlay layers in a launch with per_sm CTAs per SM: most busy warps, then
+// the shorter chunk; cl = 0 when none fits.
+TileShape widest_shape(const rrtmgp_b200_batch_t* b, int domain, int nlay, int per_sm)
 {
-    const int bin = ceil_div_i(nlay, 8);
-    TileShape s = b->shape[domain][bin];
-    if (s.cl && s.P >= 1 && s.P <= max_columns(b, domain, nlay, s.cl)) return s;
     TileShape best;
-    for (const int smem : {b->sm_smem / 2 - b->static_smem - 1024, b->max_smem}) {
-        int best_busy = -1;
-        for (int cl : {8, 16}) {
-            const int P = columns_in(b, domain, nlay, cl, smem);
-            if (P < 1) continue;
-            const int busy = P * ceil_div_i(nlay, cl);
-            if (busy > best_busy) {
-                best_busy = busy;
-                best.cl = cl;
-                best.P = P;
-            }
+    int best_busy = -1;
+    for (int cl : {8, 16}) {
+        const int P = columns_in(b, domain, nlay, cl, smem_limit(b, per_sm));
+        if (P < 1) continue;
+        const int busy = P * ceil_div_i(nlay, cl);
+        if (busy > best_busy) {
+            best_busy = busy;
+            best.cl = cl;
+            best.P = P;
         }
-        if (best.cl) break;
     }
     return best;
+}
+
+// The stored shape of (domain, bin) where it holds nlay layers, else cl = 0.
+TileShape stored_shape(const rrtmgp_b200_batch_t* b, int domain, int nlay)
+{
+    const TileShape& s = b->shape[domain][ceil_div_i(nlay, 8)];
+    return s.cl && s.P >= 1 && s.P <= max_columns(b, domain, nlay, s.cl) ? s : TileShape{};
+}
+
+// Shape of (domain, bin) for a grid of nlay layers: the stored one where it fits, else the heuristic's.
+TileShape shape_for(const rrtmgp_b200_batch_t* b, int domain, int nlay, int per_sm)
+{
+    const TileShape s = stored_shape(b, domain, nlay);
+    return s.cl ? s : widest_shape(b, domain, nlay, per_sm);
+}
+
+// CTAs per SM of a launch over the batch's items, one choice for all of them: the instance and the
+// shared memory of a launch are common to its tiles, so an item that does not fit twice leaves the
+// whole launch at one CTA per SM, and then every item needs the shape for one.
+// Two where every item has a shape for two, these hold nearly twice the warps of one CTA, and one CTA
+// leaves more than three of its 16 warps idle (both averaged over the work): 32 warps at 64
+// registers do no more than 16 at 128, but 24 do more than 12.  One against two CTAs, heuristic
+// shapes: 20 grids of 300 x 96 (12 warps) 5.14 -> 4.54 ms, 10 of 200 x 190 (12) 3.33 -> 3.11, 30 of
+// 16 - 132 x 30 - 175 (11.3) 2.76 -> 2.59; but 300 x 64 (16) 2.83 -> 2.87, 300 x 80 (15) 3.62 -> 4.27,
+// 300 x 128 (16) 2.93 -> 3.04, and with dense tables, whose shortwave fits twice only with half the
+// warps, 300 x 64 4.21 -> 5.00, 300 x 128 4.28 -> 5.00.
+// stored: a stored shape that does not fit twice means one CTA.
+constexpr double kTwoCtaWarps = 13., kTwoCtaGain = 0.55;
+int ctas_per_sm(const rrtmgp_b200_batch_t* b, bool stored)
+{
+    double work = 0., one = 0., two = 0.;   // sum of columns x layers, and that over the busy warps of an SM
+    for (const BatchItem& it : b->items) {
+        const TileShape h = widest_shape(b, it.domain, it.nlay, 2), f = widest_shape(b, it.domain, it.nlay, 1);
+        if (!h.cl || !f.cl) return 1;
+        if (stored) {
+            const TileShape s = stored_shape(b, it.domain, it.nlay);
+            if (s.cl && s.P > columns_in(b, it.domain, it.nlay, s.cl, smem_limit(b, 2))) return 1;
+        }
+        const double w = double(it.ncol) * it.nlay;
+        work += w;
+        one += w / (f.P * ceil_div_i(it.nlay, f.cl));
+        two += w / (2 * h.P * ceil_div_i(it.nlay, h.cl));
+    }
+    return work <= kTwoCtaWarps * one && two < kTwoCtaGain * one ? 2 : 1;
 }
 
 // Relative tile time used to order work when no measurement exists: the serial sweep length
@@ -340,15 +381,9 @@ BatchItem planned(const rrtmgp_b200_batch_t* b, const BatchItem& in, const TileS
     return it;
 }
 
-// CTAs per SM (the PER_SM instance) of a launch with smem bytes per CTA.
-int per_sm(const rrtmgp_b200_batch_t* b, size_t smem)
+int persistent_ctas(const rrtmgp_b200_batch_t* b, int per_sm, long long ntiles)
 {
-    return 2 * (smem + size_t(b->static_smem) + 1024) <= size_t(b->sm_smem) ? 2 : 1;
-}
-
-int persistent_ctas(const rrtmgp_b200_batch_t* b, size_t smem, long long ntiles)
-{
-    return int(std::min<long long>((long long)b->nsm * per_sm(b, smem), std::max<long long>(ntiles, 1)));
+    return int(std::min<long long>((long long)b->nsm * per_sm, std::max<long long>(ntiles, 1)));
 }
 
 void release_graph(rrtmgp_b200_batch_t* b)
@@ -414,10 +449,11 @@ int plan(rrtmgp_b200_batch_t* b)
 {
     if (!b->dirty) return RRTMGP_B200_OK;
     release_graph(b);
+    b->per_sm = ctas_per_sm(b, true);
     std::vector<std::pair<float, BatchItem>> keyed;
     keyed.reserve(b->items.size());
     for (const BatchItem& in : b->items) {
-        const TileShape s = shape_for(b, in.domain, in.nlay);
+        const TileShape s = shape_for(b, in.domain, in.nlay, b->per_sm);
         if (!s.cl) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "batch: no tile shape holds nlay = " +
                                                                 std::to_string(in.nlay));
         keyed.emplace_back(tile_cost(s, in.nlay), planned(b, in, s));
@@ -430,19 +466,19 @@ int plan(rrtmgp_b200_batch_t* b)
     for (auto& kv : keyed) b->order.push_back(kv.second);
     int st = upload(b, b->order, b->ntiles, b->smem);
     if (st) return st;
-    b->ctas = persistent_ctas(b, b->smem, b->ntiles);
+    b->ctas = persistent_ctas(b, b->per_sm, b->ntiles);
     b->dirty = false;
     return RRTMGP_B200_OK;
 }
 
 int launch_persistent(rrtmgp_b200_batch_t* b, const BatchItem* d_items, const long long* d_starts, int nitems,
-                      long long ntiles, size_t smem, cudaStream_t s)
+                      long long ntiles, size_t smem, int per_sm, cudaStream_t s)
 {
     RB_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), s), "batch: counter reset");
-    const int ctas = persistent_ctas(b, smem, ntiles);
+    const int ctas = persistent_ctas(b, per_sm, ntiles);
     const KdistView<float> klw = b->k[0] ? b->k[0]->v32 : KdistView<float>{};
     const KdistView<float> ksw = b->k[1] ? b->k[1]->v32 : KdistView<float>{};
-    const bool two = per_sm(b, smem) == 2;
+    const bool two = per_sm == 2;
     const auto kernel = b->dense ? (two ? batch_forward_kernel<true, 2> : batch_forward_kernel<true, 1>)
                                  : (two ? batch_forward_kernel<false, 2> : batch_forward_kernel<false, 1>);
     kernel<<<ctas, kBatchThreads, smem, s>>>(klw, ksw, d_items, d_starts, b->d_tile_item, nitems, b->d_counter);
@@ -577,7 +613,7 @@ int batch_create(rrtmgp_b200_kdist klw, rrtmgp_b200_cloud clw, rrtmgp_b200_kdist
                 "batch_create: kernel attribute");
     }
     for (const BatchItem& it : b->items)
-        if (!shape_for(b.get(), it.domain, it.nlay).cl)
+        if (!widest_shape(b.get(), it.domain, it.nlay, 1).cl)
             return fail(RRTMGP_B200_ERR_UNSUPPORTED, "batch_create: shared memory need too large for nlay = " +
                                                          std::to_string(it.nlay));
     if (cudaMalloc(&b->d_counter, sizeof(unsigned long long)) != cudaSuccess) {
@@ -598,6 +634,8 @@ int batch_autotune(rrtmgp_b200_batch_t* b, int reps, cudaStream_t s)
         return cuda_status(cudaGetLastError(), "batch_autotune");
     }
     int st = RRTMGP_B200_OK;
+    // every shape is timed as the batch will run it: the same CTAs per SM, and three waves of them
+    const int per_sm = ctas_per_sm(b, false);
     for (int domain = 0; domain < 2 && !st; ++domain) {
         // widest grid of each bin (then the deepest) is the sample
         std::map<int, const BatchItem*> sample;
@@ -611,14 +649,14 @@ int batch_autotune(rrtmgp_b200_batch_t* b, int reps, cudaStream_t s)
             TileShape best;
             float best_col_us = 0.f;
             for (int cl : {8, 16}) {
-                const int pmax = max_columns(b, domain, rep_item.nlay, cl);
+                const int pmax = columns_in(b, domain, rep_item.nlay, cl, smem_limit(b, per_sm));
                 for (int P = 1; P <= pmax && !st; ++P) {
                     TileShape cand;
                     cand.cl = cl;
                     cand.P = P;
                     const BatchItem it = planned(b, rep_item, cand);
                     const int tiles_per_copy = ceil_div_i(it.ncol, P);
-                    const int copies = std::min(256, std::max(1, ceil_div_i(3 * b->nsm, tiles_per_copy)));
+                    const int copies = std::min(256, std::max(1, ceil_div_i(3 * per_sm * b->nsm, tiles_per_copy)));
                     const std::vector<BatchItem> list(size_t(copies), it);
                     long long ntiles = 0;
                     size_t smem = 0;
@@ -627,7 +665,7 @@ int batch_autotune(rrtmgp_b200_batch_t* b, int reps, cudaStream_t s)
                     float ms_min = 0.f;
                     for (int r = -1; r < reps && !st; ++r) {   // r = -1: warm-up
                         cudaEventRecord(e0, s);
-                        st = launch_persistent(b, b->d_items, b->d_starts, copies, ntiles, smem, s);
+                        st = launch_persistent(b, b->d_items, b->d_starts, copies, ntiles, smem, per_sm, s);
                         cudaEventRecord(e1, s);
                         if (st) break;
                         if (cudaEventSynchronize(e1) != cudaSuccess) {
@@ -641,7 +679,7 @@ int batch_autotune(rrtmgp_b200_batch_t* b, int reps, cudaStream_t s)
                     if (st) break;
                     const float col_us = 1000.f * ms_min / float(copies * it.ncol);
                     if (!best.cl || col_us < best_col_us) {
-                        const int ctas = persistent_ctas(b, smem, ntiles);
+                        const int ctas = persistent_ctas(b, per_sm, ntiles);
                         best = cand;
                         best.tile_us = 1000.f * ms_min * float(ctas) / float(ntiles);
                         best_col_us = col_us;
@@ -690,11 +728,11 @@ extern "C" int rrtmgp_b200_batch_run(rrtmgp_b200_batch b, int mode, void* stream
     int st = plan(b);
     if (st) return st;
     if (mode == RRTMGP_B200_BATCH_PERSISTENT)
-        return launch_persistent(b, b->d_items, b->d_starts, int(b->order.size()), b->ntiles, b->smem, s);
+        return launch_persistent(b, b->d_items, b->d_starts, int(b->order.size()), b->ntiles, b->smem, b->per_sm, s);
     if (!b->exec) {
         if (!b->cap_stream) RB_CUDA(cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking), "batch graph");
         RB_CUDA(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal), "batch graph capture");
-        st = launch_persistent(b, b->d_items, b->d_starts, int(b->order.size()), b->ntiles, b->smem, b->cap_stream);
+        st = launch_persistent(b, b->d_items, b->d_starts, int(b->order.size()), b->ntiles, b->smem, b->per_sm, b->cap_stream);
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(b->cap_stream, &g);
         if (st) {
@@ -715,13 +753,20 @@ extern "C" int rrtmgp_b200_batch_autotune(rrtmgp_b200_batch b, int reps, void* s
     return batch_autotune(b, reps, as_stream(stream));
 }
 
+extern "C" int rrtmgp_b200_batch_ctas_per_sm(rrtmgp_b200_batch b, int* ctas)
+{
+    RB_CHECK_ARG(b && ctas, "batch_ctas_per_sm: null argument");
+    *ctas = ctas_per_sm(b, false);
+    return RRTMGP_B200_OK;
+}
+
 extern "C" int rrtmgp_b200_batch_get_plan(rrtmgp_b200_batch b, int domain, int bin, int* chunk, int* columns,
                                           float* tile_us)
 {
     RB_CHECK_ARG(b && chunk && columns && tile_us, "batch_get_plan: null argument");
     RB_CHECK_ARG((domain == 0 || domain == 1) && b->k[domain], "batch_get_plan: domain not in the batch");
     RB_CHECK_ARG(bin >= 1 && bin <= kMaxBins, "batch_get_plan: bin must be in 1..32");
-    const TileShape s = shape_for(b, domain, 8 * bin);
+    const TileShape s = shape_for(b, domain, 8 * bin, ctas_per_sm(b, true));
     *chunk = s.cl;
     *columns = s.P;
     *tile_us = s.tile_us;

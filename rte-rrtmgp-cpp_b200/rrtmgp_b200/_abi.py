@@ -253,6 +253,7 @@ _SIGS = {
     "rrtmgp_b200_batch_destroy": (_I, [_P]),
     "rrtmgp_b200_batch_run": (_I, [_P, _I, _P]),
     "rrtmgp_b200_batch_autotune": (_I, [_P, _I, _P]),
+    "rrtmgp_b200_batch_ctas_per_sm": (_I, [_P, c_int_p]),
     "rrtmgp_b200_batch_get_plan": (_I, [_P, _I, _I, c_int_p, c_int_p, C.POINTER(C.c_float)]),
     "rrtmgp_b200_batch_set_plan": (_I, [_P, _I, _I, _I, _I, C.c_float]),
     "rrtmgp_b200_batch_stats": (_I, [_P, C.POINTER(C.c_longlong), c_int_p, c_int_p, c_int_p, c_int_p]),

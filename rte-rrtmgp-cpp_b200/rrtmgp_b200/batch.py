@@ -10,8 +10,9 @@ compiled into another kernel).
 
 Tile shapes (chunk length, columns per CTA) per (domain, 8-layer bin) come from a built-in
 heuristic or from the autotuner, whose results can be cached in a JSON file keyed by the GPU
-name, the domain, the k-distribution's g-point count and the bin (the reference's tuner keeps
-its results in rte_rrtmgp_kernel_tuning.txt, include/tuner.h:78-182).
+name, the CTAs per SM they were timed with, the domain, the k-distribution's g-point count and the
+bin (the reference's tuner keeps its results in rte_rrtmgp_kernel_tuning.txt,
+include/tuner.h:78-182).
 """
 from __future__ import annotations
 
@@ -163,6 +164,12 @@ class Batched_forward:
                                                           C.byref(us)))
         return cl.value, cols.value, us.value
 
+    def ctas_per_sm(self) -> int:
+        """CTAs per SM that the batch's tile shapes are chosen and timed for (1 or 2)."""
+        n = C.c_int()
+        _abi.check(_abi.load().rrtmgp_b200_batch_ctas_per_sm(self.handle, C.byref(n)))
+        return n.value
+
     def set_plan(self, domain: int, b: int, chunk: int, columns: int, tile_us: float = 0.0):
         _abi.check(_abi.load().rrtmgp_b200_batch_set_plan(self.handle, domain, b, chunk, columns, float(tile_us)))
 
@@ -171,9 +178,9 @@ class Batched_forward:
 
     def autotune(self, reps: int = 3, cache=None) -> dict:
         """Tile shapes for every (domain, bin) of the batch: from `cache` (a JSON file) when it
-        holds them all for this GPU, else measured by rrtmgp_b200_batch_autotune (and written
+        holds them all for this GPU and this number of CTAs per SM, else measured by rrtmgp_b200_batch_autotune (and written
         to `cache`)."""
-        gpu = torch.cuda.get_device_name()
+        gpu = f"{torch.cuda.get_device_name()}|{self.ctas_per_sm()} per SM"
         ngpt = {LW: self.base.klw.get_ngpt(), SW: self.base.ksw.get_ngpt()}
         keys = {(d, b): cache_key(gpu, d, ngpt[d], b) for d in self.domains() for b in self.bins()}
         if cache is not None:

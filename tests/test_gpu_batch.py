@@ -1,7 +1,7 @@
 """Batched forward of uneven grids in one persistent launch (rrtmgp_b200_batch_*).
 
-Parity: with the per-grid chunk rule (longwave 16 layers per warp; shortwave 8 up to 128
-layers, else 16) the batched
+Parity: with the per-grid chunk rule (8 layers per warp up to 96 layers in the longwave and 128 in the
+shortwave, else 16) the batched
 results equal the per-grid fused launches to FP32 rounding (the same per-column code, compiled
 in another kernel, may contract multiply-adds differently: SAME_TOL), whatever the number of
 columns per CTA; the persistent launch and its graph replay agree bit for bit; every tile
@@ -47,11 +47,11 @@ def _atms(gpu, grids=GRIDS, seed=0):
 
 
 def _rule_plan(bf):
-    """The per-grid chunk rule (longwave 16; shortwave 8 up to 128 layers, else 16) with the most
-    columns per CTA that fit."""
+    """The per-grid chunk rule (8 up to 96 layers in the longwave, 128 in the shortwave, else 16) with the
+    most columns per CTA that fit."""
     for d in bf.domains():
         for b in bf.bins():
-            cl = 16 if d == 0 else (8 if b <= 16 else 16)
+            cl = 8 if b <= (12 if d == 0 else 16) else 16
             w = -(-8 * b // cl)
             for p in range(min(16 // w, 15), 0, -1):
                 try:
@@ -190,6 +190,54 @@ def test_batch_autotune_and_cache(tables, gpu, tmp_path):
                 assert torch.equal(a[dom][k], b[dom][k])
     bf.close()
     bf2.close()
+
+
+def _plan_warps(bf):
+    """{(domain, bin): busy warps of a CTA}"""
+    return {(d, b): -(-8 * b // cl) * cols for (d, b), (cl, cols, _) in bf.plan().items()}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dense,nlays,per_sm,warps", [
+    (False, [96], 2, 12),             # one CTA would leave four warps idle: two share an SM
+    (False, [64], 1, 16),             # one CTA is full
+    (False, [64, 80, 250], 1, 13),    # 250 layers do not fit twice: every grid gets the shapes for one CTA
+    (True, [64], 1, 16),              # dense tables: the shortwave fits twice with half the warps only
+    (True, [60, 64, 80, 250], 1, 13)])
+def test_batch_one_occupancy_for_the_launch(gpu, dense, nlays, per_sm, warps):
+    """The launch has one instance and one shared-memory size for all tiles: the CTAs per SM are chosen
+    for the batch and every shape for them, so a grid that does not fit twice does not leave the
+    others with half-sized tiles on a launch of one CTA per SM; the tuner keeps to them.  Values:
+    the per-grid launches of the same columns, at the kernels' bounds against FP64 (another
+    chunk length)."""
+    import torch
+    from rrtmgp_b200.batch import Batched_forward
+    from rrtmgp_b200.solver import Radiation_solver, atm_to_device
+    gases = S.ATM_GASES_DENSE if dense else S.ATM_GASES
+    base = Radiation_solver(S.make_kdist("lw", dense=dense), S.make_kdist("sw", dense=dense), S.make_cloud_luts("lw"),
+                            S.make_cloud_luts("sw"), gases)
+    atms = [atm_to_device(S.make_atmosphere(700, n, seed=n, clouds=True, trace_gases=dense), torch.float32, gpu)
+            for n in nlays]
+    nsm = torch.cuda.get_device_properties(gpu).multi_processor_count
+    bf = Batched_forward(base, atms)
+    ref = _copy(bf.run("per_grid"))
+    for tuned in (False, True):
+        if tuned:
+            bf.autotune(reps=1)
+        assert bf.ctas_per_sm() == per_sm
+        st = bf.stats()
+        assert st["ctas"] == per_sm * nsm and (st["smem_bytes"] + 1024) * per_sm <= 228 * 1024
+        if not tuned:
+            got = _plan_warps(bf)
+            assert min(got.values()) >= warps, got
+        out = _copy(bf.run("persistent"))
+        torch.cuda.synchronize()
+        for o, r in zip(out, ref):
+            for dom in r:
+                for k in r[dom]:
+                    tol = HR_TOL if k == "heating_rate" else FLUX_TOL
+                    assert float((o[dom][k] - r[dom][k]).abs().max()) < tol, f"{dom} {k}"
+    bf.close()
 
 
 @pytest.mark.gpu
