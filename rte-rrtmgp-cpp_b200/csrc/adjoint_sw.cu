@@ -1162,9 +1162,18 @@ int adjoint_sw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay,
     }
     const SwAdjOut out{g_tlay, g_h2o, g_o3, g_lwp, g_iwp, g_rel, g_rei, g_alb_dir, g_alb_dif,
                        flux_up, flux_dn, flux_dir, flux_net, heating_rate};
-    // parts of a column's groups per cluster: one CTA of this kernel per SM (255 registers), at most
-    // 8 CTAs in a cluster
-    const int parts = pair && 2 * CS <= 8 ? group_parts(ncol * CS, v.ngroups, 512, smem, k->nsm, 8 / CS) : 1;
+    const bool dense = v.max_minor_per_g > 3;
+    auto pick = [&](auto d, bool split) {
+        constexpr bool D = decltype(d)::value;
+        if (split) return with_flux ? sw_adjoint_kernel<CL, true, true, D, true> : sw_adjoint_kernel<CL, false, true, D, true>;
+        if (pair) return with_flux ? sw_adjoint_kernel<CL, true, true, D, false> : sw_adjoint_kernel<CL, false, true, D, false>;
+        return with_flux ? sw_adjoint_kernel<CL, true, false, D, false> : sw_adjoint_kernel<CL, false, false, D, false>;
+    };
+    auto kernel_of = [&](bool split) { return dense ? pick(std::true_type{}, split) : pick(std::false_type{}, split); };
+    // parts of a column's groups per cluster of at most 8 CTAs
+    const int parts = !pair || 2 * CS > 8 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
+        return residency()(kernel_of(s > 1), k->device, k->nsm, kLPC / CL * 32, smem, s * CS);
+    }, 8 / CS);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(ncol) * CS * parts);
     cfg.blockDim = dim3(kLPC / CL * 32);
@@ -1177,15 +1186,7 @@ int adjoint_sw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay,
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    const bool dense = v.max_minor_per_g > 3;
-    auto pick = [&](auto d) {
-        constexpr bool D = decltype(d)::value;
-        if (parts > 1) return with_flux ? sw_adjoint_kernel<CL, true, true, D, true> : sw_adjoint_kernel<CL, false, true, D, true>;
-        if (pair) return with_flux ? sw_adjoint_kernel<CL, true, true, D, false> : sw_adjoint_kernel<CL, false, true, D, false>;
-        return with_flux ? sw_adjoint_kernel<CL, true, false, D, false> : sw_adjoint_kernel<CL, false, false, D, false>;
-    };
-    const auto kernel = dense ? pick(std::true_type{}) : pick(std::false_type{});
-    RB_CUDA(cudaLaunchKernelEx(&cfg, kernel, v, gs, ca, ncol, nlay, CS, idx_o3, col_dry ? 0 : 1, play, plev,
+    RB_CUDA(cudaLaunchKernelEx(&cfg, kernel_of(parts > 1), v, gs, ca, ncol, nlay, CS, idx_o3, col_dry ? 0 : 1, play, plev,
                                tlay, col_dry, mu0, tsi_scaling, sfc_alb_dir, sfc_alb_dif, seed_up, seed_dn, seed_dir,
                                seed_hr, out, aer, parts),
             "sw_adjoint_kernel launch");

@@ -89,9 +89,13 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     SwGridIo io{ncol, nlay, play, plev, tlay, col_dry, mu0, tsi, alb_dir, alb_dif, up, dn, dir, net, hr, gs, ca, aer};
     // the split's exchange buffer: 6 accumulators per thread
     const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 6 * NW * 32;
-    const int parts = CS == 1 && split_smem <= 227 * 1024 ? group_parts(ncol, v.ngroups, NW * 32, split_smem, k->nsm) : 1;
+    const auto whole = pick_forward<CL, DENSE>(NW);
+    const int parts = CS > 1 || split_smem > 227 * 1024 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
+        return s == 1 ? residency()(whole, k->device, k->nsm, NW * 32, smem, 1)
+                      : residency()(sw_forward_split_kernel<CL, DENSE>, k->device, k->nsm, NW * 32, split_smem, s);
+    });
     if (CS == 1 && parts == 1) {
-        pick_forward<CL, DENSE>(NW)<<<ncol, NW * 32, smem, stream>>>(v, io);
+        whole<<<ncol, NW * 32, smem, stream>>>(v, io);
         RB_LAUNCH("sw_forward_kernel");
         return RRTMGP_B200_OK;
     }

@@ -12,8 +12,11 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <array>
 #include <cfloat>
 #include <cmath>
+#include <map>
+#include <mutex>
 
 #include "common.cuh"
 #include "rte_device.cuh"
@@ -419,19 +422,80 @@ struct SplitCtx : CtaCtx {
     }
 };
 
-// CTAs per column for a grid of ncol columns whose CTAs of `threads` threads (128 registers each)
-// and smem bytes, sharing the G groups of a column.  A CTA costs its groups and kGroupSetup more for its
-// set-up (layer state, scalings, cloud optics, launch); waves of CTAs run one after the other.
-// The split with the least waves x cost is taken when it saves more than a tenth.
-constexpr float kGroupSetup = 2.0f;   // measured 1.4 (LW) to 3 (SW) groups at 60 layers
-inline int group_parts(int ncol, int G, int threads, size_t smem, int nsm, int most = 8)
+// CTAs (cluster = 1) or clusters of a kernel that the device holds at once.  The driver is asked once per
+// launch shape: clusters do not cross the chip's GPCs, so of 444 places for CTAs only 432 or so take
+// clusters of three, and a grid of 441 such CTAs needs a second wave (147 x 40 shortwave: 65 us,
+// 45 in clusters of two).  0 when the driver has no answer.
+class Residency {
+public:
+    template <class K>
+    int operator()(K kernel, int device, int nsm, int threads, size_t smem, int cluster)
+    {
+        const std::array<size_t, 5> key{reinterpret_cast<size_t>(kernel), size_t(device), size_t(threads), smem,
+                                        size_t(cluster)};
+        std::lock_guard<std::mutex> lock(mu_);
+        const auto it = known_.find(key);
+        if (it != known_.end()) return it->second;
+        int n = 0;
+        cudaError_t e;
+        if (cluster == 1) {
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+            n *= nsm;
+        } else {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(cluster);
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = unsigned(cluster);
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        if (known_.size() >= 4096) known_.clear();   // launch shapes of many handles
+        known_[key] = n;
+        return n;
+    }
+
+private:
+    std::mutex mu_;
+    std::map<std::array<size_t, 5>, int> known_;
+};
+inline Residency& residency()
 {
-    const int per_sm = int(std::max<size_t>(1, std::min<size_t>(512 / threads, (227 * 1024) / (smem + 1024))));
-    const long slots = long(nsm) * per_sm;
-    auto cost = [&](int s) { return float((long(ncol) * s + slots - 1) / slots) * (kGroupSetup + float((G + s - 1) / s)); };
+    static Residency r;
+    return r;
+}
+
+// CTAs per column for a grid of ncol columns of G groups.  at_once(s): columns that the device holds at
+// once when s CTAs share the groups of each (0: not possible), for s = 1 in the instance that an
+// unsplit grid runs.  A CTA costs its groups and kGroupSetup more for its set-up (layer state,
+// scalings, cloud optics, launch); waves of CTAs run one after the other.  The split with the
+// least waves x cost is taken when it saves more than a tenth.
+constexpr float kGroupSetup = 2.0f;   // measured 1.4 (LW) to 3 (SW) groups at 60 layers
+template <class F>
+int group_parts(int ncol, int G, F&& at_once, int most = 8)
+{
+    const int whole = at_once(1);
+    if (whole < 1) return 1;
+    auto cost = [&](int columns, int s) {
+        return float((ncol + columns - 1) / columns) * (kGroupSetup + float((G + s - 1) / s));
+    };
+    float least = 0.9f * cost(whole, 1);
     int best = 1;
-    for (int s = 2; s <= std::min(G, most); ++s)
-        if (cost(s) < 0.9f * cost(1) && cost(s) < cost(best)) best = s;
+    for (int s = 2; s <= std::min(G, most); ++s) {
+        const int columns = at_once(s);
+        if (columns < 1 || cost(columns, s) >= least) continue;
+        least = cost(columns, s);
+        best = s;
+    }
     return best;
 }
 
