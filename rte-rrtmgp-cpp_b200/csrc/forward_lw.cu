@@ -30,16 +30,18 @@ __global__ void __launch_bounds__(512) lw_forward_cluster_kernel(const KdistView
     cooperative_groups::this_cluster().sync();   // no CTA leaves while another may store into its shared memory
 }
 
-// The instance for columns of NW chunks of 8 layers: register caps that let more CTAs share an SM, as
-// the kernel waits on table loads (16 warps per SM at 128 registers).  At 80 registers (40 bytes
-// of spill loads) an SM holds 24 warps; 9 and 10 chunks need none at 96.
+// The instance for columns of NW chunks of 8 layers whose CTAs take smem bytes: register caps that let
+// more CTAs share an SM, as the kernel waits on table loads (16 warps per SM at 128 registers).  At
+// 80 registers (40 bytes of spill loads) an SM holds 24 warps; 9 and 10 chunks need none at 96.  Only
+// where the CTAs fit and some SM gets more than one (crowded: more columns than SMs): 147 x 72 unsplit takes
+// 54 us at 128 registers, 58 at 96.
 template <int CL, bool DENSE>
-auto pick_forward(int NW) -> void (*)(const KdistView<float>, const LwGridIo)
+auto pick_forward(int NW, size_t smem, bool crowded) -> void (*)(const KdistView<float>, const LwGridIo)
 {
     if constexpr (CL == 8) {
-        if (NW <= 8) return lw_forward_kernel<CL, DENSE, 256, 3>;
-        if (NW <= 10) return lw_forward_kernel<CL, DENSE, 320, 2>;
-        if (NW <= 12) return lw_forward_kernel<CL, DENSE, 384, 2>;
+        if (crowded && NW <= 8 && ctas_fit(3, smem)) return lw_forward_kernel<CL, DENSE, 256, 3>;
+        if (crowded && NW > 8 && NW <= 10 && ctas_fit(2, smem)) return lw_forward_kernel<CL, DENSE, 320, 2>;
+        if (crowded && NW > 10 && NW <= 12 && ctas_fit(2, smem)) return lw_forward_kernel<CL, DENSE, 384, 2>;
     }
     return lw_forward_kernel<CL, DENSE>;
 }
@@ -60,8 +62,8 @@ int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_lw: shared memory need exceeds 220 KB");
     static PerDeviceOnce attr;
     int st = attr.run([] {
-        for (int nw : {8, 10, 12, 16}) {   // every instance
-            const cudaError_t e = cudaFuncSetAttribute(pick_forward<CL, DENSE>(nw),
+        for (int nw : {8, 10, 12, 16, 17}) {   // every instance
+            const cudaError_t e = cudaFuncSetAttribute(pick_forward<CL, DENSE>(nw, 0, nw < 17),
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
             if (e != cudaSuccess) return e;
         }
@@ -82,7 +84,7 @@ int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     LwGridIo io{ncol, nlay, play, plev, tlay, tlev, tsfc, col_dry, emis, up, dn, net, hr, gs, ca};
     // the split's exchange buffer: 4 accumulators per thread
     const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 4 * NW * 32;
-    const auto whole = pick_forward<CL, DENSE>(NW);
+    const auto whole = pick_forward<CL, DENSE>(NW, smem, ncol > k->nsm);
     const int parts = CS > 1 || split_smem > 227 * 1024 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
         return s == 1 ? residency()(whole, k->device, k->nsm, NW * 32, smem, 1)
                       : residency()(lw_forward_split_kernel<CL, DENSE>, k->device, k->nsm, NW * 32, split_smem, s);

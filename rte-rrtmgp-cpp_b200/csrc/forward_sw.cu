@@ -30,21 +30,27 @@ __global__ void __launch_bounds__(512) sw_forward_cluster_kernel(const KdistView
     cooperative_groups::this_cluster().sync();   // no CTA leaves while another may store into its shared memory
 }
 
-// The instance for columns of NW chunks.  The kernel waits on table loads, dependent arithmetic and the
-// chunk exchange, so more resident warps are worth some spills: at 128 registers an SM holds 16
-// warps, and 9 or 12 chunks leave a CTA alone on it.  At 96 registers (132 bytes of spill
-// loads) two CTAs of 9 or 10 chunks fit; at 80 (260) two of 11 or 12; at 64 (384) two of 13 - 16.
-// Measured against 128 registers: 1000 x 72 419 -> 313 us, 4096 x 91 1.72 -> 1.37 ms, 8192 x 128
-// 3.88 -> 3.57 ms.  Up to 8 chunks, where 15 or 16 warps fit at 128, the caps gained nothing (2000 x 60
-// 453 us, 461 at 80 registers; 2000 x 40 325 us, 324 at 96).
+// The instance for columns of NW chunks whose CTAs take smem bytes.  The kernel waits on table loads,
+// dependent arithmetic and the chunk exchange, so more resident warps are worth some spills: at 128
+// registers an SM holds 16 warps, and 9 or more chunks leave a CTA alone on it.  At 96 registers
+// (132 bytes of spill loads) two CTAs of 9 or 10 chunks share an SM; at 80 (260) two of 11 or 12; at
+// 64 (384) two of 13 - 16.  Measured against 128 registers: 1000 x 72 419 -> 313 us, 4096 x 91
+// 1.72 -> 1.37 ms, 8192 x 128 3.88 -> 3.57 ms.  Up to 8 chunks, where 15 or 16 warps fit at 128, the caps
+// gained nothing (2000 x 60 453 us, 461 at 80 registers; 2000 x 40 325 us, 324 at 96).
+// Without the second CTA the spills only cost, so a cap is taken where two CTAs fit and some SM gets
+// two (crowded: more columns than SMs); alone on its SM a CTA of 147 x 128 takes 75 us at 128 registers, 98
+// at 64.  Aerosols and dense tables exceed half an SM from 97 - 121 layers on: 600 x 128 with
+// aerosols 410 us at 128 registers, 502 at 64; dense tables 502, 614.  For 13 - 16 chunks, where the gain
+// is least, the two have to fit in 196 KB: the next shared-memory size of an SM leaves its L1
+// 28 KB instead of 60 (600 x 104 with aerosols, 2 x 102 KB: 389 us at 128 registers, 408 at 64; dense tables
+// without, 2 x 95 KB: 483, 434).
 template <int CL, bool DENSE>
-auto pick_forward(int NW) -> void (*)(const KdistView<float>, const SwGridIo)
+auto pick_forward(int NW, size_t smem, bool crowded) -> void (*)(const KdistView<float>, const SwGridIo)
 {
     if constexpr (CL == 8) {
-        if (NW <= 8) return sw_forward_kernel<CL, DENSE>;
-        if (NW <= 10) return sw_forward_kernel<CL, DENSE, 320, 2>;
-        if (NW <= 12) return sw_forward_kernel<CL, DENSE, 384, 2>;
-        return sw_forward_kernel<CL, DENSE, 512, 2>;
+        if (crowded && NW > 8 && NW <= 12 && ctas_fit(2, smem))
+            return NW <= 10 ? sw_forward_kernel<CL, DENSE, 320, 2> : sw_forward_kernel<CL, DENSE, 384, 2>;
+        if (crowded && NW > 12 && ctas_fit(2, smem, 196 * 1024)) return sw_forward_kernel<CL, DENSE, 512, 2>;
     }
     return sw_forward_kernel<CL, DENSE>;
 }
@@ -66,8 +72,8 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_sw: shared memory need exceeds 220 KB");
     static PerDeviceOnce attr;
     int st = attr.run([] {
-        for (int nw : {8, 10, 12, 16}) {   // every instance
-            const cudaError_t e = cudaFuncSetAttribute(pick_forward<CL, DENSE>(nw),
+        for (int nw : {8, 10, 12, 16, 17}) {   // every instance
+            const cudaError_t e = cudaFuncSetAttribute(pick_forward<CL, DENSE>(nw, 0, nw < 17),
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
             if (e != cudaSuccess) return e;
         }
@@ -89,7 +95,7 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     SwGridIo io{ncol, nlay, play, plev, tlay, col_dry, mu0, tsi, alb_dir, alb_dif, up, dn, dir, net, hr, gs, ca, aer};
     // the split's exchange buffer: 6 accumulators per thread
     const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 6 * NW * 32;
-    const auto whole = pick_forward<CL, DENSE>(NW);
+    const auto whole = pick_forward<CL, DENSE>(NW, smem, ncol > k->nsm);
     const int parts = CS > 1 || split_smem > 227 * 1024 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
         return s == 1 ? residency()(whole, k->device, k->nsm, NW * 32, smem, 1)
                       : residency()(sw_forward_split_kernel<CL, DENSE>, k->device, k->nsm, NW * 32, split_smem, s);

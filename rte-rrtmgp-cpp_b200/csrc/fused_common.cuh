@@ -422,6 +422,10 @@ struct SplitCtx : CtaCtx {
     }
 };
 
+// Whether per_sm CTAs of smem bytes of dynamic shared memory fit in `bytes` of an SM (each takes 1 KB
+// more than it asks for).
+inline bool ctas_fit(int per_sm, size_t smem, size_t bytes = 228 * 1024) { return per_sm * (smem + 1024) <= bytes; }
+
 // CTAs (cluster = 1) or clusters of a kernel that the device holds at once.  The driver is asked once per
 // launch shape: clusters do not cross the chip's GPCs, so of 444 places for CTAs only 432 or so take
 // clusters of three, and a grid of 441 such CTAs needs a second wave (147 x 40 shortwave: 65 us,

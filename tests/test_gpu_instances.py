@@ -1,7 +1,11 @@
-"""Which compiled instance of the kernels a call runs, in which launch, and its values.
+"""Which compiled instance of the fused forward kernels a call runs, and its values.
 
 Grids too small to fill the chip share each column's g-points between CTAs (the split kernels); the
-tests with a few dozen columns run those.  Kernel, grid and block are read from the profiler."""
+tests with a few dozen columns run those.  Here grids wide enough to run unsplit cover the
+instances that larger calls use: chunk counts up to 8, 10, 12 and 16, sparse and dense tables,
+with and without aerosols.  Instance, grid and block are read from the
+profiler (<chunk length, dense, threads, CTAs per SM>); a column sample is compared with the FP64 oracle at
+the fused kernels' bounds (5e-3 W/m2, 0.01 K/day)."""
 import json
 import re
 import tempfile
@@ -11,7 +15,11 @@ import pytest
 
 from rrtmgp_b200 import synthetic as S
 
+from test_gpu_scale import _take
+
 pytestmark = pytest.mark.gpu
+HR_TOL = 0.01
+FLUX_TOL = 5e-3
 
 
 @pytest.fixture(scope="module")
@@ -60,6 +68,13 @@ def launches(call):
     return [(m.group(1), e["args"]["grid"][0], e["args"]["block"][0]) for m, e in found if m]
 
 
+def _check(got, ref, cols, what):
+    for k in ref:
+        if k in got:
+            e = float(np.max(np.abs(got[k][:, cols].double().cpu().numpy() - ref[k])))
+            assert e < (HR_TOL if k == "heating_rate" else FLUX_TOL), f"{what} {k}: {e:.3e}"
+
+
 def test_split_leaves_no_second_wave_of_clusters(solvers, gpu):
     """147 x 40 in the shortwave: CTAs of five warps, three per SM, 444 places for 441 CTAs in clusters of three --
     but clusters do not cross GPCs, so some would wait for a second wave.  Clusters of two fit."""
@@ -68,3 +83,46 @@ def test_split_leaves_no_second_wave_of_clusters(solvers, gpu):
     fused.solve_sw(d)
     (name, ctas, threads), = launches(lambda: fused.solve_sw(d))
     assert name.startswith("sw_forward_split_kernel<8, false") and (ctas, threads) == (2 * 147, 160)
+
+
+@pytest.mark.parametrize("ncol,nlay,dense,aerosols,lw,sw", [
+    # two or three capped CTAs share an SM
+    (880, 60, False, False, "8, D, 256, 3", "8, D, 512, 1"),
+    (880, 72, False, False, "8, D, 320, 2", "8, D, 320, 2"),
+    (880, 96, False, True, "8, D, 384, 2", "8, D, 384, 2"),
+    (880, 128, False, False, "16, D, 512, 1", "8, D, 512, 2"),
+    (880, 64, True, True, "8, D, 256, 3", "8, D, 512, 1"),
+    (880, 80, True, False, "8, D, 320, 2", "8, D, 320, 2"),
+    (880, 96, True, True, "8, D, 384, 2", "8, D, 384, 2"),
+    (880, 104, True, False, "16, D, 512, 1", "8, D, 512, 2"),
+    # two shortwave CTAs do not fit, or leave the L1 too little: no cap
+    (880, 104, False, True, "16, D, 512, 1", "8, D, 512, 1"),
+    (880, 128, False, True, "16, D, 512, 1", "8, D, 512, 1"),
+    (880, 128, True, False, "16, D, 512, 1", "8, D, 512, 1"),
+    (880, 104, True, True, "16, D, 512, 1", "8, D, 512, 1"),
+    # one CTA per SM at most: no cap
+    (140, 72, False, False, "8, D, 512, 1", "8, D, 512, 1"),
+    (140, 96, True, True, "8, D, 512, 1", "8, D, 512, 1")])
+def test_forward_instance_and_values(oracle_mod, solvers, gpu, ncol, nlay, dense, aerosols, lw, sw):
+    fused, t, gases = solvers[dense]
+    atm, d = _grid(gpu, ncol, nlay, dense, aerosols, 300 + nlay)
+    out = {}
+
+    def call():
+        out["lw"] = fused.solve_lw(d)
+        out["sw"] = fused.solve_sw(d, with_aerosols=aerosols)
+
+    b = "true" if dense else "false"
+    assert [n for n, _, _ in launches(call)] == ["lw_forward_kernel<" + lw.replace("D", b) + ">",
+                                                  "sw_forward_kernel<" + sw.replace("D", b) + ">"]
+    cols = np.arange(0, ncol, max(1, ncol // 24))
+    few = _take(atm, cols)
+    extra = {}
+    if aerosols:
+        few["aerosols"] = {k: v[:, cols] for k, v in atm["aerosols"].items()}
+        few["rh"] = atm["rh"][:, cols]
+        extra = {"aerosol_tables": t["aer"], "delta_aerosol": True}
+    _check(out["lw"], oracle_mod.forward_lw(oracle_mod.GasOptics(t["lw"], gases), oracle_mod.CloudOptics(t["cloud_lw"]),
+                                            few), cols, "lw")
+    _check(out["sw"], oracle_mod.forward_sw(oracle_mod.GasOptics(t["sw"], gases), oracle_mod.CloudOptics(t["cloud_sw"]),
+                                            few, **extra), cols, "sw")
