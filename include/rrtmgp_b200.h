@@ -464,8 +464,9 @@ int rrtmgp_b200_heating_rate_from_layer_abs_f32(int ncol, int nlay, int ngpt, co
  * rates, in one kernel that keeps every (layer, g-point) quantity on chip.  Outputs
  * flux_up, flux_dn, flux_net (ncol, nlay+1) and heating_rate (ncol, nlay) [K/day].  The
  * vertical orientation is taken per column from play.  chunk: layers per warp (8 or 16;
- * 0 picks the tuned default).  Up to 16 chunks (16 * chunk layers) a column is one CTA; deeper
- * columns run on a thread-block cluster of ceil(chunks / 16) CTAs, nlay <= 128 * chunk. */
+ * 0 picks the length that takes less time for this ncol and nlay).  Up to 16 chunks (16 * chunk
+ * layers) a column is one CTA; deeper columns run on a thread-block cluster of ceil(chunks / 16)
+ * CTAs, nlay <= 128 * chunk. */
 int rrtmgp_b200_forward_lw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud cloud, int ncol, int nlay,
         const float* play, const float* plev, const float* tlay, const float* tlev,
         const float* tsfc, const float* col_dry, const rrtmgp_b200_gas_conc* gases, int ngases,

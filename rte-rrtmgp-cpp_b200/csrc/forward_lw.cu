@@ -46,22 +46,12 @@ auto pick_forward(int NW, size_t smem, bool crowded) -> void (*)(const KdistView
     return lw_forward_kernel<CL, DENSE>;
 }
 
+// Shared-memory limits of the instances on the current device, set once.
 template <int CL, bool DENSE>
-int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay, const float* play,
-                      const float* plev, const float* tlay, const float* tlev, const float* tsfc, const float* col_dry,
-                      const GasSet<float>& gs, const float* lwp, const float* iwp, const float* rel, const float* rei,
-                      const float* emis, float* up, float* dn, float* net, float* hr, cudaStream_t stream)
+int lw_forward_attributes()
 {
-    const KdistView<float>& v = k->v32;
-    const int NW = (nlay + CL - 1) / CL;
-    // more than 16 chunks: a cluster of CS CTAs of NWc warps per column
-    const int CS = (NW + 15) / 16, NWc = (NW + CS - 1) / CS;
-    RB_CHECK_ARG(CS <= 8, "forward_lw: nlay too large for the fused kernel (at most 128 chunks)");
-    const size_t smem = smem_layout(NWc * CL, v.ngas, v.nband, 1, CS * NWc, 2, CL,
-                                    v.max_group_bands * (CL == 8 ? 2 : 1), v.max_nscal, sizeof(LwRec), NWc).total;
-    if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_lw: shared memory need exceeds 220 KB");
     static PerDeviceOnce attr;
-    int st = attr.run([] {
+    return attr.run([] {
         for (int nw : {8, 10, 12, 16, 17}) {   // every instance
             const cudaError_t e = cudaFuncSetAttribute(pick_forward<CL, DENSE>(nw, 0, nw < 17),
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
@@ -73,7 +63,57 @@ int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
         return cudaFuncSetAttribute(lw_forward_cluster_kernel<CL, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     220 * 1024);
     }, "forward_lw attribute");
-    if (st) return st;
+}
+
+// Shared memory of one of the CS CTAs of a column (NWc chunks of CL layers each).
+template <int CL>
+size_t lw_forward_smem(const KdistView<float>& v, int NWc, int CS)
+{
+    return smem_layout(NWc * CL, v.ngas, v.nband, 1, CS * NWc, 2, CL, v.max_group_bands * (CL == 8 ? 2 : 1),
+                       v.max_nscal, sizeof(LwRec), NWc).total;
+}
+
+// Columns that the device holds at once, one CTA each in chunks of CL layers; 0 when they do not fit.
+template <int CL, bool DENSE>
+int lw_columns_at_once(rrtmgp_b200_kdist k, int ncol, int nlay)
+{
+    const int NW = ceil_div(nlay, CL);
+    const size_t smem = lw_forward_smem<CL>(k->v32, NW, 1);
+    if (smem > 220 * 1024 || lw_forward_attributes<CL, DENSE>()) return 0;
+    return residency()(pick_forward<CL, DENSE>(NW, smem, ncol > k->nsm), k->device, k->nsm, NW * 32, smem, 1);
+}
+
+// Default chunk length.  8 and 16 layers hold different numbers of columns at once (72 layers: 296 and
+// 444), and a wave of the latter takes 1.4 - 1.65 times one of the former, so the shorter time in whole
+// waves is taken at 1.5 (us, 8 and 16 layers: 400 x 72 121 and 97, 520 x 72 130 and 184, 520 x 60 134
+// and 99, 700 x 60 135 and 193, 400 x 112 177 and 199, 590 x 112 236 and 207; large grids 4096 x 91 1.12 and
+// 1.26 ms, 8192 x 128 3.24 and 2.93 ms).  Grids of up to one column per SM, split or not, are faster with
+// 8 up to 96 layers.  More than 128 layers need 16 to fit one CTA.
+template <bool DENSE>
+int lw_chunk(rrtmgp_b200_kdist k, int ncol, int nlay)
+{
+    if (nlay > 128) return 16;
+    if (ncol > k->nsm) {
+        const int n8 = lw_columns_at_once<8, DENSE>(k, ncol, nlay), n16 = lw_columns_at_once<16, DENSE>(k, ncol, nlay);
+        if (n8 > 0 && n16 > 0) return 2 * ceil_div(ncol, n8) <= 3 * ceil_div(ncol, n16) ? 8 : 16;
+    }
+    return nlay <= 96 ? 8 : 16;
+}
+
+template <int CL, bool DENSE>
+int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay, const float* play,
+                      const float* plev, const float* tlay, const float* tlev, const float* tsfc, const float* col_dry,
+                      const GasSet<float>& gs, const float* lwp, const float* iwp, const float* rel, const float* rei,
+                      const float* emis, float* up, float* dn, float* net, float* hr, cudaStream_t stream)
+{
+    const KdistView<float>& v = k->v32;
+    const int NW = (nlay + CL - 1) / CL;
+    // more than 16 chunks: a cluster of CS CTAs of NWc warps per column
+    const int CS = (NW + 15) / 16, NWc = (NW + CS - 1) / CS;
+    RB_CHECK_ARG(CS <= 8, "forward_lw: nlay too large for the fused kernel (at most 128 chunks)");
+    const size_t smem = lw_forward_smem<CL>(v, NWc, CS);
+    if (smem > 220 * 1024) return fail(RRTMGP_B200_ERR_UNSUPPORTED, "forward_lw: shared memory need exceeds 220 KB");
+    if (const int st = lw_forward_attributes<CL, DENSE>()) return st;
     CloudArgs ca{};
     if (c) {
         ca.L = CloudLut<float>{c->nband, c->nsize_liq, c->nsize_ice, float(c->radliq_lwr), float(c->liq_step),
@@ -142,10 +182,8 @@ int forward_lw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay,
 #define RB_LW_FWD(CLv, D)                                                                                          \
     launch_lw_forward<CLv, D>(k, c, ncol, nlay, play, plev, tlay, tlev, tsfc, col_dry, gs, lwp, iwp, rel, rei, \
                               sfc_emis, flux_up, flux_dn, flux_net, heating_rate, s)
-    // Up to 12 chunks of 8 layers the 8-layer instances fit 18 - 25 warps per SM (pick_forward):
-    // 1000 x 72 274 -> 244 us, 4096 x 91 1.26 -> 1.12 ms, dense tables 2000 x 60 626 -> 547 us.  Deeper
-    // columns are faster in 16-layer chunks (8192 x 128: 2.93 ms, 3.24 - 3.5 with 8).
-    if (chunk ? chunk == 8 : nlay <= 96) return dense ? RB_LW_FWD(8, true) : RB_LW_FWD(8, false);
+    if (chunk == 0) chunk = dense ? lw_chunk<true>(k, ncol, nlay) : lw_chunk<false>(k, ncol, nlay);
+    if (chunk == 8) return dense ? RB_LW_FWD(8, true) : RB_LW_FWD(8, false);
     return dense ? RB_LW_FWD(16, true) : RB_LW_FWD(16, false);
 #undef RB_LW_FWD
 }

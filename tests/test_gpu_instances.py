@@ -100,6 +100,10 @@ def test_split_leaves_no_second_wave_of_clusters(solvers, gpu):
     (880, 128, False, True, "16, D, 512, 1", "8, D, 512, 1"),
     (880, 128, True, False, "16, D, 512, 1", "8, D, 512, 1"),
     (880, 104, True, True, "16, D, 512, 1", "8, D, 512, 1"),
+    # longwave chunk length by waves: two of 8 layers against one of 16, three against two
+    (400, 72, False, False, "16, D, 512, 1", "8, D, 320, 2"),
+    (520, 60, True, False, "16, D, 512, 1", "8, D, 512, 1"),
+    (400, 112, False, False, "8, D, 512, 1", "8, D, 512, 2"),
     # one CTA per SM at most: no cap
     (140, 72, False, False, "8, D, 512, 1", "8, D, 512, 1"),
     (140, 96, True, True, "8, D, 512, 1", "8, D, 512, 1")])
