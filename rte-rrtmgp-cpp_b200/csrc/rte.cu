@@ -907,10 +907,12 @@ int rte_lw(rrtmgp_b200_bands b, int ncol, int nlay, int top_at_1, const T* tau, 
         }
         const dim3 grid(ceil_div(ncol, 32), b->ngpt);
         // 8-layer chunks in FP32 up to 128 layers (more warps with fewer rows in flight each measured
-        // faster than 16 at 8192 x 128) and in FP64 (88 registers, no spills; 16 layers spill) while two
-        // blocks share an SM: LW solve 1024 x 72 955 -> 913 us, 2000 x 40 1.01 -> 0.92 ms, but
-        // 1000 x 128 1.41 -> 1.46 ms
-        if (nlay <= (sizeof(T) == 4 ? 128 : 88))
+        // faster than 16 at 8192 x 128) and in FP64 (88 registers, no spills; 16 layers spill) where the
+        // 20 warps that an SM holds are nearly filled by blocks of ceil(nlay / 8): rte_lw in us, 16 -> 8 layers,
+        // 1000 x 24 125 -> 97, 1000 x 40 203 -> 146, 1000 x 72 335 -> 285, 1000 x 80 349 -> 297; but with 14,
+        // 16 or 11 warps 1000 x 56 251 -> 265, 1000 x 60 256 -> 267, 1000 x 88 472 -> 506
+        const int nw = ceil_div(nlay, 8);
+        if (sizeof(T) == 4 ? nw <= 16 : nw <= 10 && 20 / nw * nw > 16)
             lw_solver_chunked<T, 8, 512><<<grid, 32 * ceil_div(nlay, 8), 0, as_stream(stream)>>>(
                 a, tau, lay_src, lev_inc, lev_dec);
         else

@@ -130,3 +130,27 @@ def test_forward_instance_and_values(oracle_mod, solvers, gpu, ncol, nlay, dense
                                             few), cols, "lw")
     _check(out["sw"], oracle_mod.forward_sw(oracle_mod.GasOptics(t["sw"], gases), oracle_mod.CloudOptics(t["cloud_sw"]),
                                             few, **extra), cols, "sw")
+
+
+@pytest.mark.parametrize("nlay", [8, 47, 49, 56, 64, 65, 80, 81, 88, 96])
+def test_fp64_longwave_solver_chunks(oracle_mod, solvers, gpu, nlay):
+    """One angle in FP64: chunks of 8 layers where their blocks nearly fill the 20 warps of an SM (3 - 6, 9
+    or 10 chunks), else of 16; each at the edges of its range against the oracle."""
+    import torch
+    from rrtmgp_b200 import api
+    _, t, gases = solvers[False]
+    atm = S.make_atmosphere(37, nlay, seed=40 + nlay, clouds=False)
+    go = oracle_mod.GasOptics(t["lw"], gases).gas_optics_lw(atm["play"], atm["plev"], atm["tlay"], atm["tsfc"], atm["gases"],
+                                                            atm["tlev"])
+    emis = np.random.default_rng(5).uniform(0.8, 1.0, (37, 16))
+    up, dn = oracle_mod.rte_lw(t["lw"]["bnd_limits_gpt"], go["tau"], True, go, emis)
+    kd = api.Gas_optics_rrtmgp(t["lw"], gases)
+    src = {k: torch.as_tensor(v, dtype=torch.float64, device=gpu).contiguous() for k, v in go.items()}
+    e = torch.as_tensor(emis, device=gpu)
+    out = {}
+    (name, _, threads), = launches(lambda: out.update(f=api.Rte_lw.rte_lw(kd.bands, src["tau"], True, src, e)))
+    chunks = -(-nlay // 8)
+    cl = 8 if chunks <= 6 or chunks in (9, 10) else 16
+    assert name.startswith(f"lw_solver_chunked<double, {cl}, ") and threads == 32 * -(-nlay // cl)
+    for got, ref in zip(out["f"], (up, dn)):
+        np.testing.assert_allclose(got.cpu().numpy(), ref, rtol=1e-10, atol=1e-10 * np.abs(ref).max())
