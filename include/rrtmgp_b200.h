@@ -465,8 +465,14 @@ int rrtmgp_b200_heating_rate_from_layer_abs_f32(int ncol, int nlay, int ngpt, co
  * flux_up, flux_dn, flux_net (ncol, nlay+1) and heating_rate (ncol, nlay) [K/day].  The
  * vertical orientation is taken per column from play.  chunk: layers per warp (8 or 16;
  * 0 picks the length that takes less time for this ncol and nlay).  Up to 16 chunks (16 * chunk
- * layers) a column is one CTA; deeper columns run on a thread-block cluster of ceil(chunks / 16)
- * CTAs, nlay <= 128 * chunk. */
+ * layers) a column is one CTA, or, in a grid of too few columns to fill the GPU, a thread-block
+ * cluster of up to 8 CTAs that share its g-points; deeper columns run on a cluster of
+ * ceil(chunks / 16) CTAs, nlay <= 128 * chunk.
+ * The split and the chunk length follow ncol, so the last bits of a column's results depend on
+ * the grid it is computed in: another order of additions (a few ulp) where only the split
+ * differs, rounding of another chunk length (about 3e-6 of a field's norm) where the length does.
+ * The same holds for the split of the shortwave forward and of the adjoints below (gradients:
+ * 2e-5 of max(|value|, rms), o3 7e-4). */
 int rrtmgp_b200_forward_lw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud cloud, int ncol, int nlay,
         const float* play, const float* plev, const float* tlay, const float* tlev,
         const float* tsfc, const float* col_dry, const rrtmgp_b200_gas_conc* gases, int ngases,
@@ -516,8 +522,9 @@ int rrtmgp_b200_forward_sw_aer_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud cloud,
  * dependence on h2o is included.  Forward optical properties are recomputed per group of
  * 32 g-points on chip, nothing is stored between forward and adjoint.  chunk: 8 or 16
  * layers per warp (0 = 8); the k-distribution's bands must hold 16 or more g-points each.
- * One CTA per column up to 128 layers (chunk 16: up to what its shared memory holds); deeper
- * columns (chunk 8, nlay <= 512) run on a thread-block cluster of ceil(nlay / 128) CTAs. */
+ * One CTA per column up to 128 layers (few columns: a cluster of CTAs sharing its g-points, as
+ * the forward), RRTMGP_B200_ERR_UNSUPPORTED where its shared memory does not hold them; deeper
+ * columns (chunk 8, nlay <= 1024) run on a thread-block cluster of ceil(nlay / 128) CTAs. */
 int rrtmgp_b200_adjoint_lw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud cloud, int ncol, int nlay,
         const float* play, const float* plev, const float* tlay, const float* tlev,
         const float* tsfc, const float* col_dry, const rrtmgp_b200_gas_conc* gases, int ngases,

@@ -611,7 +611,7 @@ sw_adjoint_kernel(const KdistView<float> k, const GasSet<float> gs, const SwClou
         const float af = gv ? __ldg(alb_dif + gband + size_t(icol) * nband) : 0.f;
 
         // Records (forward and derivative) of every (layer, band) of the group.  With PAIR, the
-        // records of groups gg and gg + 1 are built together at even gg into two buffers: with
+        // records of groups gg and gg + 1 are built together at every other gg into two buffers: with
         // 8 layers and 2 bands a group has 16 records per warp, so one group alone leaves half
         // the lanes idle.
         SwRec* const recs = recs0 + (PAIR ? par : 0) * kLPC * mgb;

@@ -112,7 +112,6 @@ struct KdistView {
     // Fused-kernel metadata: g-points are processed in groups of 32 (one per lane).
     int ngroups;                    // ceil(ngpt / 32)
     int max_group_bands;            // most bands touched by one group
-    int max_band_minor;             // most minor intervals in one (band, atmosphere)
     const int* group_band0;         // [ngroups] first band of each group
     // Corner-packed copies for the FP32 kernels (NULL in the FP64 view):
     //   kmaj4/pfrac4 [t][p][eta][g], p < npres, eta < neta-1: (k(e,p), k(e+1,p), k(e,p+1), k(e+1,p+1))
@@ -126,7 +125,7 @@ struct KdistView {
     //   minor_g[a]   [g]: x = number of intervals covering g, y/z/w = the first three codes
     //                (c << kScalBits) | sid, c = contributor, sid = scaling kind of the
     //                interval (below); unused slots repeat y (0 when no interval covers g).
-    //   minor_gx[a]  [g][minor_gx_stride]: codes 4, 5, ... of g (NULL when no g-point has
+    //   minor_gx[a]  [g][minor_gx_stride]: codes 4, 5, ... of g (one unused entry when no g-point has
     //                more than three intervals).
     // Fused kernels (lanes = the g-points of a group of 32): the minor-interval coefficients by
     // g-point, in aligned rows that a warp reads with one load per row,

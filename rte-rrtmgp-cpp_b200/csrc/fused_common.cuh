@@ -36,8 +36,10 @@ struct __align__(16) LayerState {
 //
 // Longwave: only what the weights cannot be formed from (the major and the Planck weights are
 // products of fm, fpress and col_mix, a dozen multiplies per lane of a kernel whose FMA pipe is a
-// quarter used), because shared memory held by records is taken from the L1 that holds the
-// table rows: with 144-byte records a third of the table sectors missed it.
+// quarter used), because shared memory held by records is taken from the L1 that holds the table
+// rows.  With the aligned minor rows: 8192 x 128 3.05 -> 2.96 ms, dense tables 2000 x 60 728 -> 631 us;
+// but grids that leave an SM with 7 to 10 warps of 16 layers are slower (1000 x 104 359 -> 371 us,
+// 2000 x 160 1.24 -> 1.27 ms).
 struct __align__(16) LwRec {
     int4 kb;          // x, y: element offsets (row * ngpt) of the kmp8 rows of (t0, p0, e0) and
                       //       (t1, p0, e1); z, w: kmin4 rows of (a, t0, e0), (a, t1, e1), unit 0
@@ -537,17 +539,6 @@ __device__ __forceinline__ void setup_layer_range(const KdistView<float>& k, con
         s.pad2 = 0.f;
         st[jl] = s;
     }
-}
-
-// The whole column (layers 0 .. nlay - 1, cg stride nlay).
-__device__ __forceinline__ void setup_layers(const KdistView<float>& k, const GasSet<float>& gs, int ncol,
-                                             int nlay, int icol, bool top_at_1, const float* __restrict__ play,
-                                             const float* __restrict__ plev, const float* __restrict__ tlay,
-                                             const float* __restrict__ tlev, const float* __restrict__ col_dry,
-                                             LayerState* st, float* cg, int tid, int nthr)
-{
-    setup_layer_range(k, gs, ncol, nlay, icol, top_at_1, play, plev, tlay, tlev, col_dry, st, cg, nlay, 0, nlay, tid,
-                      nthr);
 }
 
 // Table layouts the corner-packed FP32 kernels take: minor intervals inside one band (their

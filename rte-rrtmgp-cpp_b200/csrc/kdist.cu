@@ -235,15 +235,11 @@ int fill_view(rrtmgp_b200_kdist_t* k, KdistView<T>& v, const rrtmgp_b200_kdist_t
         kmin[atm] = conv<T>(m.kminor.data(), m.kminor.size());
         a.add(kmin[atm], &v.kminor[atm]);
     }
-    int in_band = 1, max_minor = 0;
-    for (int atm = 0; atm < 2; ++atm) {
+    int in_band = 1;
+    for (int atm = 0; atm < 2; ++atm)
         for (size_t i = 0; i < mh[atm].gstart.size(); ++i)
             if (g2b[mh[atm].gstart[i]] != g2b[mh[atm].gend[i] - 1]) in_band = 0;
-        for (int b = 0; b < t->nband; ++b)
-            max_minor = std::max(max_minor, mh[atm].band_begin[b + 1] - mh[atm].band_begin[b]);
-    }
     v.minor_in_band = in_band;
-    v.max_band_minor = max_minor;
     // Scaling kinds (see KdistView): one per distinct (minor gas, scaling gas, complement
     // flag) among the density-scaled intervals and per minor gas among the others.
     std::vector<int> sid[2], sgas_k[2], ssg_k[2], sfl_k[2];

@@ -14,6 +14,7 @@ import pytest
 from rrtmgp_b200 import synthetic as S
 
 from test_gpu_adjoint import _check, _fd, _fd_bands, _get, _informative, _seeds, _sw_seeds
+from test_gpu_instances import launches
 from test_gpu_scale import _take
 from test_gpu_stages import N, T, cmp, dtypes
 
@@ -164,6 +165,33 @@ def test_sw_adjoint_dense_matches_fd(oracle_mod, dense, gpu):
     for key in ("tlay", "h2o", "o3"):
         _check(f"dense sw d/d{key}", got[key], _fd(fwd, atm, seeds, key), _informative(_get(atm, key)))
     _check("dense sw d/dsfc_alb_dir", got["sfc_alb_dir"], _fd_bands(fwd, atm, seeds, "sfc_alb_dir"))
+
+
+def test_adjoints_dense_unsplit_match_fd(oracle_mod, dense, gpu):
+    """The dense tables' adjoints on a grid that is not split (two columns are, in the tests above):
+    the gradients of three sampled columns against central differences."""
+    import torch
+    from rrtmgp_b200.autodiff import adjoint_lw, adjoint_sw
+    from rrtmgp_b200.solver import atm_to_device
+    rng = np.random.default_rng(31)
+    ncol, nlay, cols = 900, 20, [0, 451, 899]
+    atm = S.make_atmosphere(ncol, nlay, seed=98, clouds=True, trace_gases=True)
+    few, d = _take(atm, cols), atm_to_device(atm, torch.float32, gpu)
+    base, fused = _solvers(dense)
+    for dom, keys, seeds in (("lw", ("tlay", "tsfc", "h2o"), _seeds(nlay, ncol, rng)),
+                             ("sw", ("tlay", "h2o"), _sw_seeds(nlay, ncol, rng))):
+        kd, cl = oracle_mod.GasOptics(dense[dom], GASES), oracle_mod.CloudOptics(dense["cloud_" + dom])
+        fwd = oracle_mod.forward_lw if dom == "lw" else oracle_mod.forward_sw
+        t = {k: torch.as_tensor(v, dtype=torch.float32, device=gpu).contiguous() for k, v in seeds.items()}
+        out = {}
+        names = [n for n, _, _ in launches(lambda: out.update(
+            adjoint_lw(fused, d, t["flux_up"], t["flux_dn"], t["heating_rate"]) if dom == "lw" else
+            adjoint_sw(fused, d, t["flux_up"], t["flux_dn"], t["flux_dn_dir"], t["heating_rate"])))]
+        assert len(names) == 1 and names[0].startswith(dom + "_adjoint_kernel<8, ") and names[0].endswith("true, false>")
+        part = {k: np.ascontiguousarray(v[:, cols]) for k, v in seeds.items()}
+        for k in keys:
+            ref = _fd(lambda a: fwd(kd, cl, a), few, part, k)
+            _check(f"dense {dom} unsplit d/d{k}", out[k].double().cpu().numpy()[..., cols], ref, _informative(_get(few, k)))
 
 
 def test_batched_dense_matches_oracle(oracle_mod, dense, gpu):
