@@ -673,14 +673,16 @@ int launch_lw_adjoint(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
         ca.lwp = lwp; ca.iwp = iwp; ca.rel = rel; ca.rei = rei;
         ca.present = 1;
     }
-    const int parts = CS > 1 || CL != 8 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
-        return s == 1 ? residency()(lw_adjoint_kernel<CL, false, FLUX, DENSE>, k->device, k->nsm, NWc * 32, smem, 1)
-                      : residency()(lw_adjoint_kernel<8, false, FLUX, DENSE, true>, k->device, k->nsm, NWc * 32, smem, s);
-    });
+    const auto whole = lw_adjoint_kernel<CL, false, FLUX, DENSE>;
+    const auto ask = [&](int s) {
+        return s == 1 ? resident(whole, k->nsm, NWc * 32, smem, 1)
+                      : resident(lw_adjoint_kernel<8, false, FLUX, DENSE, true>, k->nsm, NWc * 32, smem, s);
+    };
+    const int parts =
+        CS > 1 || CL != 8 ? 1 : group_parts(ncol, v.ngroups, residency()(whole, k->device, NWc * 32, smem, ask));
     if (CS == 1 && parts == 1) {
-        lw_adjoint_kernel<CL, false, FLUX, DENSE><<<ncol, NWc * 32, smem, stream>>>(v, gs, ca, ncol, nlay, 1, idx_o3, col_dry ? 0 : 1,
-                                                                  play, plev, tlay, tlev, tsfc, col_dry, emis, su, sd,
-                                                                  sh, out, 1);
+        whole<<<ncol, NWc * 32, smem, stream>>>(v, gs, ca, ncol, nlay, 1, idx_o3, col_dry ? 0 : 1, play, plev, tlay, tlev,
+                                                tsfc, col_dry, emis, su, sd, sh, out, 1);
         RB_LAUNCH("lw_adjoint_kernel");
         return RRTMGP_B200_OK;
     }

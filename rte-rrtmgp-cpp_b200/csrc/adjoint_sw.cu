@@ -1170,10 +1170,12 @@ int adjoint_sw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nlay,
         return with_flux ? sw_adjoint_kernel<CL, true, false, D, false> : sw_adjoint_kernel<CL, false, false, D, false>;
     };
     auto kernel_of = [&](bool split) { return dense ? pick(std::true_type{}, split) : pick(std::false_type{}, split); };
-    // parts of a column's groups per cluster of at most 8 CTAs
-    const int parts = !pair || 2 * CS > 8 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
-        return residency()(kernel_of(s > 1), k->device, k->nsm, kLPC / CL * 32, smem, s * CS);
-    }, 8 / CS);
+    // parts of a column's groups per cluster of at most 8 CTAs (the launch shape is told by CS)
+    const auto ask = [&](int s) {
+        return s * CS > 8 ? 0 : resident(kernel_of(s > 1), k->nsm, kLPC / CL * 32, smem, s * CS);
+    };
+    const int parts = !pair || 2 * CS > 8 ? 1 : group_parts(ncol, v.ngroups,
+                                                            residency()(kernel_of(false), k->device, CS, smem, ask));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(ncol) * CS * parts);
     cfg.blockDim = dim3(kLPC / CL * 32);

@@ -80,7 +80,7 @@ int lw_columns_at_once(rrtmgp_b200_kdist k, int ncol, int nlay)
     const int NW = ceil_div(nlay, CL);
     const size_t smem = lw_forward_smem<CL>(k->v32, NW, 1);
     if (smem > 220 * 1024 || lw_forward_attributes<CL, DENSE>()) return 0;
-    return residency()(pick_forward<CL, DENSE>(NW, smem, ncol > k->nsm), k->device, k->nsm, NW * 32, smem, 1);
+    return resident(pick_forward<CL, DENSE>(NW, smem, ncol > k->nsm), k->nsm, NW * 32, smem, 1);
 }
 
 // Default chunk length.  8 and 16 layers hold different numbers of columns at once (72 layers: 296 and
@@ -125,10 +125,12 @@ int launch_lw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     // the split's exchange buffer: 4 accumulators per thread
     const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 4 * NW * 32;
     const auto whole = pick_forward<CL, DENSE>(NW, smem, ncol > k->nsm);
-    const int parts = CS > 1 || split_smem > 227 * 1024 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
-        return s == 1 ? residency()(whole, k->device, k->nsm, NW * 32, smem, 1)
-                      : residency()(lw_forward_split_kernel<CL, DENSE>, k->device, k->nsm, NW * 32, split_smem, s);
-    });
+    const auto ask = [&](int s) {
+        return s == 1 ? resident(whole, k->nsm, NW * 32, smem, 1)
+                      : resident(lw_forward_split_kernel<CL, DENSE>, k->nsm, NW * 32, split_smem, s);
+    };
+    const int parts = CS > 1 || split_smem > 227 * 1024
+                          ? 1 : group_parts(ncol, v.ngroups, residency()(whole, k->device, NW * 32, smem, ask));
     if (CS == 1 && parts == 1) {
         whole<<<ncol, NW * 32, smem, stream>>>(v, io);
         RB_LAUNCH("lw_forward_kernel");

@@ -96,10 +96,12 @@ int launch_sw_forward(rrtmgp_b200_kdist k, rrtmgp_b200_cloud c, int ncol, int nl
     // the split's exchange buffer: 6 accumulators per thread
     const size_t xch = align16(smem), split_smem = xch + sizeof(double) * 6 * NW * 32;
     const auto whole = pick_forward<CL, DENSE>(NW, smem, ncol > k->nsm);
-    const int parts = CS > 1 || split_smem > 227 * 1024 ? 1 : group_parts(ncol, v.ngroups, [&](int s) {
-        return s == 1 ? residency()(whole, k->device, k->nsm, NW * 32, smem, 1)
-                      : residency()(sw_forward_split_kernel<CL, DENSE>, k->device, k->nsm, NW * 32, split_smem, s);
-    });
+    const auto ask = [&](int s) {
+        return s == 1 ? resident(whole, k->nsm, NW * 32, smem, 1)
+                      : resident(sw_forward_split_kernel<CL, DENSE>, k->nsm, NW * 32, split_smem, s);
+    };
+    const int parts = CS > 1 || split_smem > 227 * 1024
+                          ? 1 : group_parts(ncol, v.ngroups, residency()(whole, k->device, NW * 32, smem, ask));
     if (CS == 1 && parts == 1) {
         whole<<<ncol, NW * 32, smem, stream>>>(v, io);
         RB_LAUNCH("sw_forward_kernel");

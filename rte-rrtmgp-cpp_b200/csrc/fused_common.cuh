@@ -428,78 +428,84 @@ struct SplitCtx : CtaCtx {
 // more than it asks for).
 inline bool ctas_fit(int per_sm, size_t smem, size_t bytes = 228 * 1024) { return per_sm * (smem + 1024) <= bytes; }
 
-// CTAs (cluster = 1) or clusters of a kernel that the device holds at once.  The driver is asked once per
-// launch shape: clusters do not cross the chip's GPCs, so of 444 places for CTAs only 432 or so take
-// clusters of three, and a grid of 441 such CTAs needs a second wave (147 x 40 shortwave: 65 us,
-// 45 in clusters of two).  0 when the driver has no answer.
-class Residency {
+// CTAs (cluster = 1) or clusters of a kernel that the device holds at once, by the driver; 0 when it has
+// no answer.  Clusters do not cross the chip's GPCs: of 444 places for CTAs only 432 or so take clusters
+// of three, and a grid of 441 such CTAs needs a second wave (147 x 40 shortwave: 65 us, 42 in
+// clusters of two).
+template <class K>
+int resident(K kernel, int nsm, int threads, size_t smem, int cluster)
+{
+    int n = 0;
+    cudaError_t e;
+    if (cluster == 1) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+        n *= nsm;
+    } else {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cluster);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(cluster);
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+    }
+    if (e == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
+}
+
+// Columns that the device holds at once when s = 1 .. 8 CTAs share the groups of each ([s]; [0] unused).
+using AtOnce = std::array<int, 9>;
+
+// The AtOnce of a launch shape (kernel, device, threads, shared memory), asked from the driver once: eight
+// questions take longer than a small grid's launch.
+class ResidencyTable {
 public:
-    template <class K>
-    int operator()(K kernel, int device, int nsm, int threads, size_t smem, int cluster)
+    template <class K, class F>
+    AtOnce operator()(K kernel, int device, int threads, size_t smem, F&& ask)
     {
-        const std::array<size_t, 5> key{reinterpret_cast<size_t>(kernel), size_t(device), size_t(threads), smem,
-                                        size_t(cluster)};
+        const std::array<size_t, 4> key{reinterpret_cast<size_t>(kernel), size_t(device), size_t(threads), smem};
         std::lock_guard<std::mutex> lock(mu_);
         const auto it = known_.find(key);
         if (it != known_.end()) return it->second;
-        int n = 0;
-        cudaError_t e;
-        if (cluster == 1) {
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
-            n *= nsm;
-        } else {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(cluster);
-            cfg.blockDim = dim3(threads);
-            cfg.dynamicSmemBytes = smem;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = unsigned(cluster);
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-        }
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            n = 0;
-        }
-        if (known_.size() >= 4096) known_.clear();   // launch shapes of many handles
-        known_[key] = n;
-        return n;
+        AtOnce a{};
+        for (int s = 1; s <= 8; ++s) a[s] = ask(s);
+        if (known_.size() >= 1024) known_.clear();   // launch shapes of many handles
+        known_[key] = a;
+        return a;
     }
 
 private:
     std::mutex mu_;
-    std::map<std::array<size_t, 5>, int> known_;
+    std::map<std::array<size_t, 4>, AtOnce> known_;
 };
-inline Residency& residency()
+inline ResidencyTable& residency()
 {
-    static Residency r;
+    static ResidencyTable r;
     return r;
 }
 
-// CTAs per column for a grid of ncol columns of G groups.  at_once(s): columns that the device holds at
-// once when s CTAs share the groups of each (0: not possible), for s = 1 in the instance that an
-// unsplit grid runs.  A CTA costs its groups and kGroupSetup more for its set-up (layer state,
+// CTAs per column for a grid of ncol columns of G groups, at[s] columns at once (0: not possible; s = 1 in
+// the instance that an unsplit grid runs).  A CTA costs its groups and kGroupSetup more for its set-up (layer state,
 // scalings, cloud optics, launch); waves of CTAs run one after the other.  The split with the
 // least waves x cost is taken when it saves more than a tenth.
 constexpr float kGroupSetup = 2.0f;   // measured 1.4 (LW) to 3 (SW) groups at 60 layers
-template <class F>
-int group_parts(int ncol, int G, F&& at_once, int most = 8)
+inline int group_parts(int ncol, int G, const AtOnce& at)
 {
-    const int whole = at_once(1);
-    if (whole < 1) return 1;
-    auto cost = [&](int columns, int s) {
-        return float((ncol + columns - 1) / columns) * (kGroupSetup + float((G + s - 1) / s));
+    if (at[1] < 1) return 1;
+    auto cost = [&](int s) {
+        return float((ncol + at[s] - 1) / at[s]) * (kGroupSetup + float((G + s - 1) / s));
     };
-    float least = 0.9f * cost(whole, 1);
+    float least = 0.9f * cost(1);
     int best = 1;
-    for (int s = 2; s <= std::min(G, most); ++s) {
-        const int columns = at_once(s);
-        if (columns < 1 || cost(columns, s) >= least) continue;
-        least = cost(columns, s);
+    for (int s = 2; s <= std::min(G, 8); ++s) {
+        if (at[s] < 1 || cost(s) >= least) continue;
+        least = cost(s);
         best = s;
     }
     return best;

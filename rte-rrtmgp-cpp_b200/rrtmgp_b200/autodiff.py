@@ -45,7 +45,7 @@ class _LongwaveFn(torch.autograd.Function):
         clouds = lwp is not None
         # outputs of its own, not copies of the solver's; no zeros for outputs without a gradient
         nlay, ncol = static["play"].shape
-        out = fused.solve_lw(atm, with_clouds=clouds, out=fused.new_outputs("lw", static["play"], ncol, nlay))
+        out = fused._run_lw(atm, clouds, fused.new_outputs("lw", static["play"], ncol, nlay), ncol, nlay)
         res = tuple(out[k] for k in ("flux_up", "flux_dn", "flux_net", "heating_rate"))
         ctx.set_materialize_grads(False)
         ctx.fused, ctx.atm, ctx.clouds = fused, atm, clouds
@@ -196,7 +196,7 @@ class _ShortwaveFn(torch.autograd.Function):
         atm["gases"] = gases
         clouds = lwp is not None
         nlay, ncol = static["play"].shape
-        out = fused.solve_sw(atm, with_clouds=clouds, out=fused.new_outputs("sw", static["play"], ncol, nlay))
+        out = fused._run_sw(atm, clouds, False, fused.new_outputs("sw", static["play"], ncol, nlay), ncol, nlay)
         res = tuple(out[k] for k in ("flux_up", "flux_dn", "flux_dn_dir", "flux_net", "heating_rate"))
         ctx.set_materialize_grads(False)
         ctx.fused, ctx.atm, ctx.clouds = fused, atm, clouds

@@ -170,6 +170,10 @@ class Radiation_solver:
         return {k: b[k] for k in ("flux_up", "flux_dn", "flux_dn_dir", "flux_net", "heating_rate")}
 
 
+# level fluxes that a fused solve writes; heating rates come beside them
+_LEVEL_OUTPUTS = {"lw": ("flux_up", "flux_dn", "flux_net"), "sw": ("flux_up", "flux_dn", "flux_net", "flux_dn_dir")}
+
+
 class Fused_solver:
     """FP32 column forward through the fused kernels (rrtmgp_b200_forward_lw_f32 / _sw_f32):
     same inputs and outputs as Radiation_solver.solve_lw / solve_sw, no g-point arrays."""
@@ -190,20 +194,16 @@ class Fused_solver:
     @staticmethod
     def new_outputs(kind, like, ncol, nlay):
         """Output tensors of one solve ("lw" or "sw")."""
-        return {k: torch.empty(shape, dtype=torch.float32, device=like.device)
-                for k, shape in Fused_solver._output_shapes(kind, ncol, nlay)}
-
-    @staticmethod
-    def _output_shapes(kind, ncol, nlay):
-        names = ("flux_up", "flux_dn", "flux_net") + (("flux_dn_dir",) if kind == "sw" else ())
-        return [(k, (nlay + 1, ncol)) for k in names] + [("heating_rate", (nlay, ncol))]
+        o = {k: torch.empty((nlay + 1, ncol), dtype=torch.float32, device=like.device) for k in _LEVEL_OUTPUTS[kind]}
+        o["heating_rate"] = torch.empty((nlay, ncol), dtype=torch.float32, device=like.device)
+        return o
 
     @staticmethod
     def _check_outputs(kind, out, like, ncol, nlay):
         """out, if it holds every output as the kernels write it; they see only addresses, so a short
         or FP64 tensor would be written past its end."""
-        for k, shape in Fused_solver._output_shapes(kind, ncol, nlay):
-            t = out.get(k)
+        for k in _LEVEL_OUTPUTS[kind] + ("heating_rate",):
+            t, shape = out.get(k), (nlay + (k != "heating_rate"), ncol)
             if (t is None or t.shape != shape or t.dtype != torch.float32 or t.device != like.device
                     or not t.is_contiguous()):
                 raise ValueError(f"out[{k!r}]: a contiguous float32 tensor of shape {shape} on {like.device} is needed")
@@ -211,12 +211,17 @@ class Fused_solver:
 
     def solve_lw(self, atm: dict, with_clouds: bool = True, out: dict | None = None):
         """out: tensors to write instead of the solver's own (new_outputs); others raise ValueError."""
-        from . import _abi
         play = atm["play"]
-        assert play.dtype == torch.float32, "the fused path is FP32"
         nlay, ncol = play.shape
         o = (self._outputs("lw", play, ncol, nlay) if out is None
              else self._check_outputs("lw", out, play, ncol, nlay))
+        return self._run_lw(atm, with_clouds, o, ncol, nlay)
+
+    def _run_lw(self, atm, with_clouds, o, ncol, nlay):
+        """solve_lw into o, outputs made here (new_outputs) or checked."""
+        from . import _abi
+        play = atm["play"]
+        assert play.dtype == torch.float32, "the fused path is FP32"
         P = api._ptr
         arr, keep = api.Gas_optics_rrtmgp._gases(atm["gases"], ncol, nlay, atm["play"])
         c = self.base.clw if (with_clouds and self.base.clw is not None) else None
@@ -233,12 +238,17 @@ class Fused_solver:
         """with_aerosols: atm["aerosols"] {aermr01 .. aermr11} and atm["rh"] (nlay, ncol) through
         the base solver's aerosol tables, inside the fused kernel (rrtmgp_b200_forward_sw_aer_f32).
         out: as solve_lw."""
-        from . import _abi
         play = atm["play"]
-        assert play.dtype == torch.float32, "the fused path is FP32"
         nlay, ncol = play.shape
         o = (self._outputs("sw", play, ncol, nlay) if out is None
              else self._check_outputs("sw", out, play, ncol, nlay))
+        return self._run_sw(atm, with_clouds, with_aerosols, o, ncol, nlay)
+
+    def _run_sw(self, atm, with_clouds, with_aerosols, o, ncol, nlay):
+        """solve_sw into o, as _run_lw."""
+        from . import _abi
+        play = atm["play"]
+        assert play.dtype == torch.float32, "the fused path is FP32"
         P = api._ptr
         arr, keep = api.Gas_optics_rrtmgp._gases(atm["gases"], ncol, nlay, atm["play"])
         c = self.base.csw if (with_clouds and self.base.csw is not None) else None
