@@ -524,7 +524,7 @@ int rrtmgp_b200_forward_sw_aer_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud cloud,
  * layers per warp (0 = 8); the k-distribution's bands must hold 16 or more g-points each.
  * One CTA per column up to 128 layers (few columns: a cluster of CTAs sharing its g-points, as
  * the forward), RRTMGP_B200_ERR_UNSUPPORTED where its shared memory does not hold them; deeper
- * columns (chunk 8, nlay <= 1024) run on a thread-block cluster of ceil(nlay / 128) CTAs. */
+ * columns (chunk 8, nlay <= 512) run on a thread-block cluster of ceil(nlay / 128) CTAs. */
 int rrtmgp_b200_adjoint_lw_f32(rrtmgp_b200_kdist k, rrtmgp_b200_cloud cloud, int ncol, int nlay,
         const float* play, const float* plev, const float* tlay, const float* tlev,
         const float* tsfc, const float* col_dry, const rrtmgp_b200_gas_conc* gases, int ngases,
