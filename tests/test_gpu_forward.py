@@ -258,7 +258,7 @@ def test_fused_forward_group_split(tables, gpu, ncol, nlay):
     for solve in (fused.solve_lw, fused.solve_sw):
         whole, split = {}, {}
         names = [n for n, _, _ in launches(lambda: (whole.update({k: v[:, :ncol].clone() for k, v in solve(a).items()}),
-                                                    split.update(solve(b))))]
+                                                    split.update(solve(b))), 2)]
         assert "_forward_kernel" in names[0] and "_forward_split_kernel" in names[1], names
         for k, w in whole.items():
             scale = w.abs().clamp_min(1e-3 * float(w.abs().max()))
