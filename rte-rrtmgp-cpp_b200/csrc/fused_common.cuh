@@ -38,8 +38,8 @@ struct __align__(16) LayerState {
 // products of fm, fpress and col_mix, a dozen multiplies per lane of a kernel whose FMA pipe is a
 // quarter used), because shared memory held by records is taken from the L1 that holds the table
 // rows.  With the aligned minor rows: 8192 x 128 3.05 -> 2.96 ms, dense tables 2000 x 60 728 -> 631 us;
-// but grids that leave an SM with 7 to 10 warps of 16 layers are slower (1000 x 104 359 -> 371 us,
-// 2000 x 160 1.24 -> 1.27 ms).
+// but grids that leave an SM with 7 to 10 warps of 16 layers are 1 - 2.5% slower (1000 x 104 359 -> 363 us,
+// 600 x 104 261 -> 268, 1000 x 160 620 -> 625).
 struct __align__(16) LwRec {
     int4 kb;          // x, y: element offsets (row * ngpt) of the kmp8 rows of (t0, p0, e0) and
                       //       (t1, p0, e1); z, w: kmin4 rows of (a, t0, e0), (a, t1, e1), unit 0
@@ -260,9 +260,19 @@ __device__ __forceinline__ void load_rows(const GasTab& k, const int4& kb, int g
         r.m0 = ldg4_if(k.kmin4 + (kb.z + g), nmax > 0);
         r.m1 = ldg4_if(k.kmin4 + (kb.w + g), nmax > 0);
     }
-    constexpr int n1 = SW ? 1 : 2;   // intervals in unit 0
-    r.n0 = ldg4_if(k.kmin4 + (kb.z + k.ngpt + g), nmax > n1);
-    r.n1 = ldg4_if(k.kmin4 + (kb.w + k.ngpt + g), nmax > n1);
+    if constexpr (SW) {   // one interval in unit 0
+        r.n0 = ldg4_if(k.kmin4 + (kb.z + k.ngpt + g), nmax > 1);
+        r.n1 = ldg4_if(k.kmin4 + (kb.w + k.ngpt + g), nmax > 1);
+    } else {
+        // Two in unit 0.  A branch, taken by few warps: with predicated loads the longwave forward was 2 - 4%
+        // slower (300 x 104 180 us, 173 now; 1000 x 112 389, 380; 147 x 160 96.5, 94.7; 8192 x 128 2.94 ms,
+        // 2.89).  Unit 0, which most warps read, is better predicated (1000 x 128 400 us, 426 with a branch).
+        r.n0 = r.n1 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (nmax > 2) {
+            r.n0 = __ldg(k.kmin4 + (kb.z + k.ngpt + g));
+            r.n1 = __ldg(k.kmin4 + (kb.w + k.ngpt + g));
+        }
+    }
 }
 
 // The (T, eta) corners in fminor order of the first and the second pair of two rows.
